@@ -1,0 +1,54 @@
+"""The prefill GEMM at the edges of its tiles: W rows around a CTA's 128 and a pair's 256, tokens around the multiples of 32 a tile is
+made of and the 256 / 512 an accumulator or two hold, K of one block and of block counts that splits divide unevenly.
+
+The reference is the fp64 product of the operands as rounded to the 16-bit type; the fp32 accumulation may differ from it by
+(cols + 4) * 2^-24 * sum|h(W) h(x)| (the reference's bound for its own GEMM, tests/unit/vulkan/test_vk_head.cpp:1005-1013)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from halo_b200 import backend as hb
+from halo_b200 import capi, synth
+
+pytestmark = pytest.mark.gpu
+GUARD = 12  # floats behind every y row that must stay as they were
+
+
+@pytest.fixture(scope="module")
+def be():
+    return hb.CudaBackend(0)
+
+
+def rounded(a: np.ndarray, bf16: bool) -> np.ndarray:
+    if not bf16:
+        return a.astype(np.float16).astype(np.float64)
+    u = np.ascontiguousarray(a, np.float32).view(np.uint32).astype(np.uint64)
+    u = (u + 0x7FFF + ((u >> 16) & 1)) >> 16 << 16
+    return u.astype(np.uint32).view(np.float32).astype(np.float64)
+
+
+@pytest.mark.parametrize("t", (synth.Q4_K, synth.Q6_K, synth.Q8_0, synth.Q4_0))
+@pytest.mark.parametrize("bf16", (False, True))
+@pytest.mark.parametrize("m,n,k", [(1, 1, 256), (33, 129, 512), (64, 128, 2816), (97, 257, 4352), (255, 40, 512), (257, 513, 768), (513, 384, 1024), (700, 2000, 512)])
+def test_gemm_tile_edges(be, checker, t, bf16, m, n, k):
+    st = be.create_stream()
+    w, x = synth.quant_weights(t, n, k, 80 + m, 1), synth.activations(m, k, 80 + m, 2)
+    wb = raw = be.import_host_readonly(np.ascontiguousarray(w).view(np.uint8).reshape(-1))
+    variant = capi.GEMM_TCGEN05_BF16 if bf16 else capi.GEMM_TCGEN05_F16
+    if t != synth.Q4_K:
+        wb, variant = be.repack(st, t, hb.TensorRef.of(raw), n, k), capi.GEMM_TCGEN05_BF16_R if bf16 else capi.GEMM_TCGEN05_F16_R
+    xb, yb, stride = be.import_host_readonly(x), be.allocate(m * (n + GUARD) * 4), (n + GUARD) * 4
+    got = []
+    for _ in range(2):  # a second call finds the counters and partial sums as the first one left them
+        be.upload(st, hb.TensorRef.of(yb), np.full(m * (n + GUARD), -77.0, np.float32))
+        be.gemv(st, hb.GemvArgs(t, hb.TensorRef.of(wb), hb.TensorRef.of(xb), hb.TensorRef(yb, 0, 0, stride), n, k, m, variant, allow_gemm=True))
+        y = np.empty((m, n + GUARD), np.float32)
+        be.download(st, hb.TensorRef.of(yb), y)
+        st.wait()
+        got.append(y)
+    assert np.array_equal(got[0], got[1])
+    assert np.all(got[0][:, n:] == -77.0)
+    hw, hx = rounded(checker.dequantize(t, w, n * k).reshape(n, k), bf16), rounded(x, bf16)
+    err = np.abs(got[0][:, :n].astype(np.float64) - hx @ hw.T)
+    assert np.all(err <= (k + 4) * 2.0**-24 * (np.abs(hx) @ np.abs(hw).T))
