@@ -238,7 +238,7 @@ int run_gemv(HaloCudaCtx* ctx, const GemvCall& c, uint32_t requested, cudaStream
         case HALO_CUDA_GEMV_EXACT8: return launch_gemv_exact8(c, s);
         case HALO_CUDA_GEMV_WARP_F32:
             if (!gemv_warp_f32_supports(c)) return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: gemv_warp_f32 does not take this weight type");
-            return launch_gemv_warp_f32(c, s);
+            return launch_gemv_warp_f32(ctx, c, s);
         case HALO_CUDA_GEMV_MMA_F16X2:
             if (!gemv_mma_supports(c))
                 return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: gemv_mma_f16x2 needs Q4_K weights in dense 16-byte-aligned rows");

@@ -1,4 +1,5 @@
-// gemv_warp_f32: the fp32 CUDA-core streaming kernel for decode-shaped calls, all four block formats.
+// gemv_warp_f32: the fp32 CUDA-core streaming kernel for decode-shaped calls, all four block formats.  Q4_K rows, and raw rows of the
+// other formats whose K is too long for gemv_raw.cu's shared memory, run the kernel below; the rest runs there.
 //
 // One warp owns one W row.  The row is cut into 16- or 32-weight chunks; lane L takes chunks L, L+32, ... so a
 // warp-wide load walks the row front to back in runs of whole sectors.  Inside a chunk the sub-block scale is
@@ -262,7 +263,8 @@ bool gemv_warp_f32_supports(const GemvCall& c) {
     }
 }
 
-int launch_gemv_warp_f32(const GemvCall& c, cudaStream_t s) {
+int launch_gemv_warp_f32(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
+    if (gemv_raw_supports(c)) return launch_gemv_raw(ctx, c, s);
     switch (c.wtype) {
         case HALO_CUDA_T_Q4_0: return launch_t<HALO_CUDA_T_Q4_0>(c, s);
         case HALO_CUDA_T_Q8_0: return launch_t<HALO_CUDA_T_Q8_0>(c, s);
