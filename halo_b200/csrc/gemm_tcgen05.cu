@@ -255,7 +255,7 @@ __device__ __forceinline__ uint32_t bytes02(uint32_t w) { return __byte_perm(w, 
 __device__ __forceinline__ uint32_t bytes13(uint32_t w) { return __byte_perm(w, 0x64646464u, 0x4341); }
 
 struct GemmQ4K {  // raw rows of 144-byte super-blocks: quarter j = sub-blocks 2j (low nibbles) and 2j + 1 (high)
-    static constexpr uint32_t kBlock = 144;
+    static constexpr uint32_t kBlock = 144, kPitch = 144;
     static constexpr double kConvertNs = 350.0;  // to convert a stage
     struct Regs {
         uint4 h, q[2];
@@ -303,7 +303,7 @@ struct GemmQ4K {  // raw rows of 144-byte super-blocks: quarter j = sub-blocks 2
 };
 
 struct GemmQ80R {  // repacked groups of 272 B: d[8] fp16 | chunk c < 4, thread t < 4: words (block 2c, step 0/1), (block 2c+1, step 0/1)
-    static constexpr uint32_t kBlock = 272;
+    static constexpr uint32_t kBlock = 272, kPitch = 272;
     static constexpr double kConvertNs = 320.0;
     struct Regs {
         uint4 w[4];  // thread t: (block 2j, step 0), (2j, 1), (2j + 1, 0), (2j + 1, 1)
@@ -339,7 +339,7 @@ struct GemmQ80R {  // repacked groups of 272 B: d[8] fp16 | chunk c < 4, thread 
 };
 
 struct GemmQ40R {  // repacked groups of 144 B: d[8] fp16 | chunk c < 2, thread t < 4: the quant word (bytes 4t..4t+3) of blocks 4c..4c+3
-    static constexpr uint32_t kBlock = 144;
+    static constexpr uint32_t kBlock = 144, kPitch = 144;
     static constexpr double kConvertNs = 310.0;
     struct Regs {
         uint2 w[4];  // thread t's words of blocks 2j and 2j + 1: low nibbles = weights 4t.., high nibbles = weights 16 + 4t..
@@ -376,7 +376,9 @@ struct GemmQ40R {  // repacked groups of 144 B: d[8] fp16 | chunk c < 2, thread 
 };
 
 struct GemmQ6KR {  // repacked groups of 224 B: scales[16] int8 | d fp16, pad | half n < 2, thread t < 4: ql words (b, lh) | thread t: qh words (n, lh)
-    static constexpr uint32_t kBlock = 224;
+    // A slot row holds 16 bytes of the next group as well: at a pitch of 224 bytes (an even number of 16-byte units) the 16-byte loads of
+    // eight rows met on four bank groups.
+    static constexpr uint32_t kBlock = 224, kPitch = 240;
     static constexpr double kConvertNs = 475.0;
     struct Regs {
         uint4 ql[4];     // thread t: words (b 0, lh 0), (0, 1), (1, 0), (1, 1) of half j / 2
@@ -399,11 +401,15 @@ struct GemmQ6KR {  // repacked groups of 224 B: scales[16] int8 | d fp16, pad | 
     }
     template <bool BF16>
     __device__ static __forceinline__ void emit(const Regs& r, uint32_t j, uint8_t* dst, uint32_t sw) {
+        if (j & 1u) emit_half<BF16, 1>(r, dst, sw);
+        else emit_half<BF16, 0>(r, dst, sw);
+    }
+    /// Runs 2 J and 2 J + 1 of a 128-weight half: ql words b = 0, 1, their nibbles J; qh bits 4 J + 2 b and + 1 of every byte.
+    template <bool BF16, int J>
+    __device__ static __forceinline__ void emit_half(const Regs& r, uint8_t* dst, uint32_t sw) {
         const float d = __half2float(__ushort_as_half(static_cast<uint16_t>(r.d)));
-        const uint32_t nib = 4u * (j & 1u);
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {          // runs 2 (j % 2) + b of 32 weights: ql words b, bits 2 (2 (j % 2) + b) of qh
-            const uint32_t hsh = nib + 2u * b;  // the run's two bits of every qh byte start at this bit
+        for (int b = 0; b < 2; ++b) {
 #pragma unroll
             for (int g = 0; g < 4; ++g) {  // weights 8g .. 8g+7 of the run: lh = g / 2, threads 2 (g % 2) and + 1
                 const int lh = g >> 1;
@@ -415,7 +421,8 @@ struct GemmQ6KR {  // repacked groups of 224 B: scales[16] int8 | d fp16, pad | 
                     const uint4& l4 = r.ql[2 * (g & 1) + k];
                     const uint2& h2 = r.qh[2 * (g & 1) + k];
                     const uint32_t l = b ? (lh ? l4.w : l4.z) : (lh ? l4.y : l4.x), h = lh ? h2.y : h2.x;
-                    const uint32_t w = ((l >> nib) & 0x0F0F0F0Fu) | (((h >> hsh) & 0x03030303u) << 4);
+                    const uint32_t hi = J ? (b ? h >> 2 : h) : (b ? h << 2 : h << 4);  // the run's two bits at bits 4 and 5 of every byte
+                    const uint32_t w = ((l >> (4 * J)) & 0x0F0F0F0Fu) | (hi & 0x30303030u);
                     // (d*s)*(q-32): 19-bit scale x 6-bit code is exact in fp32, rounded once to 16 bits
                     v[2 * k] = pack2<BF16>(mul2(ds2, widen(codes(bytes02(w), 32))));
                     v[2 * k + 1] = pack2<BF16>(mul2(ds2, widen(codes(bytes13(w), 32))));
@@ -441,7 +448,7 @@ template <bool BF16, class F>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap, const __grid_constant__ GemmArgs a) {
     extern __shared__ uint8_t smem_raw[];
-    constexpr uint32_t kRawTile = kCtaRows * F::kBlock;
+    constexpr uint32_t kRawTile = kCtaRows * F::kPitch;
     // tiles need 1024-byte alignment (one swizzle atom)
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     const uint32_t tiles = smem_u32(smem);
@@ -601,7 +608,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
                 ok = g_mbar_wait_warp(raw_full(rw.slot), rw.parity);
                 if (!ok) break;
                 typename F::Regs regs;
-                F::load(regs, smem + raw_off + rw.slot * kRawTile + r * F::kBlock, j);
+                F::load(regs, smem + raw_off + rw.slot * kRawTile + r * F::kPitch, j);
                 // The slot may be refilled once every lane's words are in registers: the vote cannot be taken before (an arrival behind the
                 // load instructions alone let the copy engine overwrite the first rows of a slow warp).
                 const uint32_t others = __ballot_sync(0xFFFFFFFFu, F::fold(regs) != 0x9E3779B9u);
@@ -744,7 +751,7 @@ struct GemmPlan {
 
 template <class F>
 void ring_sizes(GemmPlan* p) {
-    const uint32_t raw = kCtaRows * F::kBlock, stage = kTileW + p->nacc * (p->nt / 2u) * (kBK * 2u);
+    const uint32_t raw = kCtaRows * F::kPitch, stage = kTileW + p->nacc * (p->nt / 2u) * (kBK * 2u);
     p->raw_slots = 2;
     p->stages = std::min((kSmemTiles - 2u * raw) / stage, kMaxStages);
     if (p->stages * stage + 3u * raw <= kSmemTiles) p->raw_slots = 3;
@@ -804,7 +811,7 @@ int launch_t(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
                            CU_TENSOR_MAP_SWIZZLE_128B, "x", &xmap))
         return rc;
     // (the pitch of a one-row matrix is never used, but has to be a valid one)
-    if (int rc = encode_2d(CU_TENSOR_MAP_DATA_TYPE_UINT32, c.w, c.row_bytes / 4u, c.rows, std::max(c.w_stride, c.row_bytes), F::kBlock / 4u, kCtaRows,
+    if (int rc = encode_2d(CU_TENSOR_MAP_DATA_TYPE_UINT32, c.w, c.row_bytes / 4u, c.rows, std::max(c.w_stride, c.row_bytes), F::kPitch / 4u, kCtaRows,
                            CU_TENSOR_MAP_SWIZZLE_NONE, "the weight matrix", &wmap))
         return rc;
     cudaLaunchAttribute attr[1];
