@@ -61,8 +61,8 @@ struct GemmArgs {
     uint32_t rows, n_vec, nb;
     uint32_t nt, nacc;       // tokens per accumulator, accumulators per tile
     uint32_t stages, raw_slots;
-    uint32_t token_tiles, splits, units;
-    float* partials;         // splits > 1: [tile][split][CTA of the pair][nacc * nt tokens][128 rows]
+    uint32_t token_tiles, whole, splits, units;  // units: tiles [0, whole) over all of K, then `splits` shares of K of every further tile
+    float* partials;         // splits > 1: [tile - whole][split][CTA of the pair][nacc * nt tokens][128 rows]
     uint32_t* error_word;
 };
 
@@ -379,7 +379,7 @@ struct GemmQ6KR {  // repacked groups of 224 B: scales[16] int8 | d fp16, pad | 
     // A slot row holds 16 bytes of the next group as well: at a pitch of 224 bytes (an even number of 16-byte units) the 16-byte loads of
     // eight rows met on four bank groups.
     static constexpr uint32_t kBlock = 224, kPitch = 240;
-    static constexpr double kConvertNs = 475.0;
+    static constexpr double kConvertNs = 380.0;
     struct Regs {
         uint4 ql[4];     // thread t: words (b 0, lh 0), (0, 1), (1, 0), (1, 1) of half j / 2
         uint2 qh[4];     // thread t: words (lh 0, lh 1)
@@ -504,10 +504,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
     };
     auto unit_of = [&](uint32_t u) {
         Unit r;
-        r.split = u % a.splits, r.tile = u / a.splits;
+        r.tile = u, r.split = 0, r.sb0 = 0, r.sb1 = a.nb;
+        if (u >= a.whole && a.splits > 1) {
+            r.tile = a.whole + (u - a.whole) / a.splits, r.split = (u - a.whole) % a.splits;
+            r.sb0 = static_cast<uint32_t>(uint64_t{a.nb} * r.split / a.splits);
+            r.sb1 = static_cast<uint32_t>(uint64_t{a.nb} * (r.split + 1) / a.splits);
+        }
         r.t_tile = r.tile % a.token_tiles, r.w_tile = r.tile / a.token_tiles;
-        r.sb0 = static_cast<uint32_t>(uint64_t{a.nb} * r.split / a.splits);
-        r.sb1 = static_cast<uint32_t>(uint64_t{a.nb} * (r.split + 1) / a.splits);
         return r;
     };
 
@@ -635,7 +638,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
             const uint32_t row = un.w_tile * kPairRows + rank * kCtaRows + quarter * 32u + lane;
             const uint32_t tile_tokens = a.nacc * a.nt;
             const uint64_t part_floats = uint64_t{tile_tokens} * kCtaRows;
-            float* part = a.partials + (uint64_t{un.tile} * a.splits * 2u + rank) * part_floats + quarter * 32u + lane;
+            const bool shared = a.splits > 1 && un.tile >= a.whole;  // this unit is a share of its tile's K
+            float* part = shared ? a.partials + ((uint64_t{un.tile - a.whole} * a.splits + un.split) * 2u + rank) * part_floats + quarter * 32u + lane : nullptr;
             for (uint32_t acc = 0; acc < a.nacc; ++acc) {
                 const uint32_t which = ac.slot + acc;
                 ok = g_mbar_wait_warp(acc_full(which), ac.parity);
@@ -647,8 +651,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
                     uint32_t v[32];
                     HC_TMEM_LD32(v, tmem_base + ((quarter * 32u) << 16) + which * 256u + c);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (a.splits > 1) {
-                        float* p = part + uint64_t{un.split} * 2u * part_floats + uint64_t{acc * a.nt + c} * kCtaRows;
+                    if (shared) {
+                        float* p = part + uint64_t{acc * a.nt + c} * kCtaRows;
 #pragma unroll
                         for (uint32_t k = 0; k < 32u; ++k) p[k * kCtaRows] = __uint_as_float(v[k]);
                     } else if (row < a.rows) {
@@ -687,21 +691,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
     cluster_sync();
 }
 
-/// y = the splits' partial sums added in split order.  grid (128-row halves of the W tiles, tokens / 8), 32 x 4 threads: a lane takes four
-/// consecutive W rows of two tokens.  (The last CTA to finish a tile adding them itself had 128 threads' loads in flight for what the whole
-/// device does here.)
+/// y of the split tiles = their partial sums added in split order.  grid (128-row halves of the tiles from `whole` on, tokens / 8), 32 x 4
+/// threads: a lane takes four consecutive W rows of two tokens.  (The last CTA to finish a tile adding them itself had 128 threads' loads in
+/// flight for what the whole device does here.)
 __global__ void __launch_bounds__(128) add_splits_kernel(const float* __restrict__ partials, float* __restrict__ y, uint64_t y_stride, uint32_t rows, uint32_t n_vec,
-                                                         uint32_t tile_tokens, uint32_t token_tiles, uint32_t splits) {
+                                                         uint32_t tile_tokens, uint32_t token_tiles, uint32_t whole, uint32_t splits) {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const uint32_t half = blockIdx.x, r = (threadIdx.x & 31u) * 4u, row = half * kCtaRows + r;
+    const uint32_t rest = blockIdx.x >> 1, half = blockIdx.x & 1u, w_tile = (whole + rest) / token_tiles, t_tile = (whole + rest) % token_tiles;
+    const uint32_t r = (threadIdx.x & 31u) * 4u, row = w_tile * kPairRows + half * kCtaRows + r;
     const uint64_t part_floats = uint64_t{tile_tokens} * kCtaRows;
 #pragma unroll
     for (uint32_t u = 0; u < 2; ++u) {
-        const uint32_t t = blockIdx.y * 8u + u * 4u + (threadIdx.x >> 5);
+        const uint32_t in = blockIdx.y * 8u + u * 4u + (threadIdx.x >> 5), t = t_tile * tile_tokens + in;
         if (t >= n_vec) break;
-        const uint64_t tile = uint64_t{half >> 1} * token_tiles + t / tile_tokens;
-        const float* p = partials + (tile * splits * 2u + (half & 1u)) * part_floats + uint64_t{t % tile_tokens} * kCtaRows + r;
+        const float* p = partials + (uint64_t{rest} * splits * 2u + half) * part_floats + uint64_t{in} * kCtaRows + r;
         float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll 4
         for (uint32_t s = 0; s < splits; ++s) {
@@ -747,6 +751,7 @@ int encode_2d(CUtensorMapDataType type, const void* base, uint64_t inner, uint64
 /// How a call is cut into units of (256 W rows, T tokens, a share of K).
 struct GemmPlan {
     uint32_t nt, nacc, stages, raw_slots, w_tiles, token_tiles, splits;
+    uint64_t whole, units;  // tiles over all of K; units of work
 };
 
 template <class F>
@@ -759,10 +764,12 @@ void ring_sizes(GemmPlan* p) {
 
 /// The cheapest (T, splits) by a model of the measured times (ns): a K step of 64 costs 1.42 a token for its MMAs and the format's
 /// conversion, which overlap but for the issue slots and the shared memory they compete for (the fourth-power mean fits T from 64 to 448);
-/// storing a tile's y costs 31 a token, under the next tile's MMAs where T <= 256; a split stores and adds 2 x 4 bytes an output.
+/// storing a tile's y costs 31 a token, under the next tile's MMAs where T <= 256.  Every pair gets as many whole tiles as there are for
+/// all; the K of the tiles left over is split, and a split stores and adds 2 x 4 bytes an output.
 template <class F>
 GemmPlan plan_gemm(uint32_t rows, uint32_t cols, uint32_t n_vec, uint32_t pairs, bool may_split) {
     const uint32_t nb = cols / 256u, w_tiles = (rows + kPairRows - 1) / kPairRows;
+    const double reread = 0.3 * (double(rows) * nb * F::kBlock / 6000.0);  // what a further token tile's pass over W (in L2) costs beyond its conversion
     GemmPlan best{};
     double best_cost = 0;
     for (uint32_t t = 32; t <= 448; t += t < 256 ? 32 : 64) {
@@ -773,14 +780,16 @@ GemmPlan plan_gemm(uint32_t rows, uint32_t cols, uint32_t n_vec, uint32_t pairs,
         if (p.stages < kMinStages) break;
         const double mma = 1.42 * t, a = mma * mma, b = F::kConvertNs * F::kConvertNs, step = std::sqrt(std::sqrt(a * a + b * b));
         const double store = 31.0 * std::min(t, n_vec);
-        for (uint32_t s = 1; s <= (may_split ? std::min(nb, 16u) : 1u); ++s) {
-            p.splits = s;
-            const uint64_t units = uint64_t{w_tiles} * p.token_tiles * s, waves = (units + pairs - 1) / pairs;
-            const double main = step * 4.0 * ((nb + s - 1) / s);
-            double cost = p.nacc == 1 ? waves * std::max(main, store) + store : waves * (main + store);
-            if (s > 1) cost += 3000.0 + 8.0 * s * n_vec * rows / 5000.0;
+        auto waves_of = [&](uint64_t waves, uint32_t blocks) {
+            const double main = step * 4.0 * blocks;
+            return waves * (p.nacc == 1 ? std::max(main, store) : main + store);
+        };
+        const uint64_t tiles = uint64_t{w_tiles} * p.token_tiles, whole = tiles / pairs * pairs, rest = tiles - whole;
+        for (uint32_t s = 1; s <= (may_split && rest != 0 ? std::min(nb, 16u) : 1u); ++s) {
+            p.splits = s, p.whole = s > 1 ? whole : tiles, p.units = p.whole + (s > 1 ? rest * s : 0);
+            double cost = waves_of(whole / pairs, nb) + waves_of((rest * s + pairs - 1) / pairs, (nb + s - 1) / s) + store + reread * p.token_tiles;
+            if (s > 1) cost += 3000.0 + 8.0 * s * rest * kPairRows * std::min(t, n_vec) / 5000.0;
             if (best_cost == 0 || cost < best_cost) best_cost = cost, best = p;
-            if (units >= 4u * uint64_t{pairs}) break;  // finer cuts only add traffic
         }
         if (t >= n_vec) break;  // nothing but padding beyond this
     }
@@ -799,13 +808,13 @@ template <bool BF16, class F>
 int launch_t(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
     const uint32_t pairs_max = static_cast<uint32_t>(ctx->prop.multiProcessorCount) / 2u;
     const GemmPlan p = plan_gemm<F>(c.rows, c.cols, c.n_vec, pairs_max, (c.flags & HALO_CUDA_GEMV_FLAG_NO_SCRATCH) == 0);
-    const uint64_t tiles = uint64_t{p.w_tiles} * p.token_tiles, units = tiles * p.splits;
-    if (units > 0x7FFFFFFFu) return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: %u x %u outputs exceed the launch limit", c.n_vec, c.rows);
+    const uint64_t rest = uint64_t{p.w_tiles} * p.token_tiles - p.whole;
+    if (p.units > 0x7FFFFFFFu) return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: %u x %u outputs exceed the launch limit", c.n_vec, c.rows);
     void* ws = nullptr;
     if (int rc = workspace(ctx, 0, uint64_t{c.n_vec} * c.cols * 2, s, &ws)) return rc;
     void* partials = nullptr;
     if (p.splits > 1)
-        if (int rc = workspace(ctx, 3, units * p.nacc * p.nt * kPairRows * 4u, s, &partials)) return rc;
+        if (int rc = workspace(ctx, 3, rest * p.splits * p.nacc * p.nt * kPairRows * 4u, s, &partials)) return rc;
     CUtensorMap xmap, wmap;
     if (int rc = encode_2d(BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, ws, c.cols, c.n_vec, uint64_t{c.cols} * 2, kBK, p.nt / 2u,
                            CU_TENSOR_MAP_SWIZZLE_128B, "x", &xmap))
@@ -820,13 +829,13 @@ int launch_t(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
     HC_CUDA(cudaLaunchKernelEx(&cast_cfg, cast_x_kernel<BF16>, c.x, c.x_stride, static_cast<uint16_t*>(ws), c.n_vec, c.cols));
     auto kern = gemm_tcgen05_kernel<BF16, F>;
     if (int rc = allow_dynamic_smem(ctx, reinterpret_cast<const void*>(kern), kGemmSmem)) return rc;
-    const GemmArgs args{c.y, c.y_stride, c.rows, c.n_vec, c.cols / 256u, p.nt, p.nacc, p.stages, p.raw_slots, p.token_tiles, p.splits, static_cast<uint32_t>(units),
+    const GemmArgs args{c.y, c.y_stride, c.rows, c.n_vec, c.cols / 256u, p.nt, p.nacc, p.stages, p.raw_slots, p.token_tiles, static_cast<uint32_t>(p.whole), p.splits, static_cast<uint32_t>(p.units),
                         static_cast<float*>(partials), ctx->error_word_dev};
-    const cudaLaunchConfig_t cfg = dependent_launch(dim3(2u * static_cast<uint32_t>(std::min<uint64_t>(units, pairs_max))), kGemmThreads, kGemmSmem, s, attr);
+    const cudaLaunchConfig_t cfg = dependent_launch(dim3(2u * static_cast<uint32_t>(std::min<uint64_t>(p.units, pairs_max))), kGemmThreads, kGemmSmem, s, attr);
     HC_CUDA(cudaLaunchKernelEx(&cfg, kern, xmap, wmap, args));
     if (p.splits > 1) {
-        const cudaLaunchConfig_t add_cfg = dependent_launch(dim3(2u * p.w_tiles, (c.n_vec + 7u) / 8u), 128, 0, s, attr);
-        HC_CUDA(cudaLaunchKernelEx(&add_cfg, add_splits_kernel, static_cast<const float*>(partials), c.y, c.y_stride, c.rows, c.n_vec, p.nacc * p.nt, p.token_tiles, p.splits));
+        const cudaLaunchConfig_t add_cfg = dependent_launch(dim3(2u * static_cast<uint32_t>(rest), p.nacc * p.nt / 8u), 128, 0, s, attr);
+        HC_CUDA(cudaLaunchKernelEx(&add_cfg, add_splits_kernel, static_cast<const float*>(partials), c.y, c.y_stride, c.rows, c.n_vec, p.nacc * p.nt, p.token_tiles, static_cast<uint32_t>(p.whole), p.splits));
     }
     return 0;
 }
