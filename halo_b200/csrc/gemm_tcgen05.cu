@@ -158,8 +158,8 @@ __device__ __forceinline__ bool elect_one() {
 struct RingPos {
     uint32_t slot, parity;
     __device__ __forceinline__ void advance(uint32_t by, uint32_t n) {
-        slot += by;
-        while (slot >= n) slot -= n, parity ^= 1u;
+        slot += by;  // by <= n
+        if (slot >= n) slot -= n, parity ^= 1u;
     }
 };
 
@@ -248,8 +248,9 @@ __device__ __forceinline__ uint32_t scaled_pair(__half2 q, __half2 d16, uint64_t
     if constexpr (BF16) return pack2<true>(mul2(d32, widen(q)));
     return as_u32(__hmul2(d16, q));
 }
-__device__ __forceinline__ void store_chunk(uint8_t* dst, uint32_t pos, uint32_t sw, const uint4& v) {
-    *reinterpret_cast<uint4*>(dst + ((pos ^ sw) << 4)) = v;
+/// Chunk `pos` of a 128-byte swizzled row; `at` is the shared-memory address of the row's chunk 0, whose bits 4-6 hold the row's xor.
+__device__ __forceinline__ void store_chunk(uint32_t at, uint32_t pos, const uint4& v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at ^ (pos << 4)), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 __device__ __forceinline__ uint32_t bytes02(uint32_t w) { return __byte_perm(w, 0x64646464u, 0x4240); }  // halves 1024 + byte 0, 1024 + byte 2
 __device__ __forceinline__ uint32_t bytes13(uint32_t w) { return __byte_perm(w, 0x64646464u, 0x4341); }
@@ -267,7 +268,7 @@ struct GemmQ4K {  // raw rows of 144-byte super-blocks: quarter j = sub-blocks 2
         r.q[1] = *reinterpret_cast<const uint4*>(row + 32 + j * 32);
     }
     template <bool BF16>
-    __device__ static __forceinline__ void emit(const Regs& r, uint32_t j, uint8_t* dst, uint32_t sw) {
+    __device__ static __forceinline__ void emit(const Regs& r, uint32_t j, uint32_t at) {
         // 6-bit codes of sub-blocks 2j (low nibbles) and 2j+1 (high nibbles), src/tensor/quant.cpp:236-244
         const uint32_t s0 = r.h.y, s1 = r.h.z, s2 = r.h.w;
         uint32_t sc0, mn0, sc1, mn1;
@@ -296,8 +297,8 @@ struct GemmQ4K {  // raw rows of 144-byte super-blocks: quarter j = sub-blocks 2
                 lo[k] = pack2<BF16>(fma2(dl, widen(codes((u & 0x000F000Fu) | 0x64006400u, 0)), ml));
                 hi[k] = pack2<BF16>(fma2(dh, widen(codes((u & 0x00F000F0u) | 0x64006400u, 0)), mh));
             }
-            store_chunk(dst, c, sw, make_uint4(lo[0], lo[1], lo[2], lo[3]));
-            store_chunk(dst, c + 4, sw, make_uint4(hi[0], hi[1], hi[2], hi[3]));
+            store_chunk(at, c, make_uint4(lo[0], lo[1], lo[2], lo[3]));
+            store_chunk(at, c + 4, make_uint4(hi[0], hi[1], hi[2], hi[3]));
         }
     }
 };
@@ -316,7 +317,7 @@ struct GemmQ80R {  // repacked groups of 272 B: d[8] fp16 | chunk c < 4, thread 
         r.d = *reinterpret_cast<const uint32_t*>(row + 4 * j);
     }
     template <bool BF16>
-    __device__ static __forceinline__ void emit(const Regs& r, uint32_t, uint8_t* dst, uint32_t sw) {
+    __device__ static __forceinline__ void emit(const Regs& r, uint32_t, uint32_t at) {
         const __half2 dd = as_half2(r.d);
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
@@ -332,7 +333,7 @@ struct GemmQ80R {  // repacked groups of 272 B: d[8] fp16 | chunk c < 4, thread 
                     v[2 * k] = scaled_pair<BF16>(codes(bytes02(w), 128), d16, d32);
                     v[2 * k + 1] = scaled_pair<BF16>(codes(bytes13(w), 128), d16, d32);
                 }
-                store_chunk(dst, 4 * b + g, sw, make_uint4(v[0], v[1], v[2], v[3]));
+                store_chunk(at, 4 * b + g, make_uint4(v[0], v[1], v[2], v[3]));
             }
         }
     }
@@ -354,7 +355,7 @@ struct GemmQ40R {  // repacked groups of 144 B: d[8] fp16 | chunk c < 2, thread 
         r.d = *reinterpret_cast<const uint32_t*>(row + 4 * j);
     }
     template <bool BF16>
-    __device__ static __forceinline__ void emit(const Regs& r, uint32_t, uint8_t* dst, uint32_t sw) {
+    __device__ static __forceinline__ void emit(const Regs& r, uint32_t, uint32_t at) {
         const __half2 dd = as_half2(r.d);
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
@@ -369,7 +370,7 @@ struct GemmQ40R {  // repacked groups of 144 B: d[8] fp16 | chunk c < 2, thread 
                     const uint32_t u = (b ? w2.y : w2.x) >> (8 * (k & 1) + (g < 2 ? 0 : 4));
                     v[k] = scaled_pair<BF16>(codes((u & 0x000F000Fu) | 0x64006400u, 8), d16, d32);
                 }
-                store_chunk(dst, 4 * b + g, sw, make_uint4(v[0], v[1], v[2], v[3]));
+                store_chunk(at, 4 * b + g, make_uint4(v[0], v[1], v[2], v[3]));
             }
         }
     }
@@ -400,13 +401,13 @@ struct GemmQ6KR {  // repacked groups of 224 B: scales[16] int8 | d fp16, pad | 
         r.d = *reinterpret_cast<const uint16_t*>(row + 16);
     }
     template <bool BF16>
-    __device__ static __forceinline__ void emit(const Regs& r, uint32_t j, uint8_t* dst, uint32_t sw) {
-        if (j & 1u) emit_half<BF16, 1>(r, dst, sw);
-        else emit_half<BF16, 0>(r, dst, sw);
+    __device__ static __forceinline__ void emit(const Regs& r, uint32_t j, uint32_t at) {
+        if (j & 1u) emit_half<BF16, 1>(r, at);
+        else emit_half<BF16, 0>(r, at);
     }
     /// Runs 2 J and 2 J + 1 of a 128-weight half: ql words b = 0, 1, their nibbles J; qh bits 4 J + 2 b and + 1 of every byte.
     template <bool BF16, int J>
-    __device__ static __forceinline__ void emit_half(const Regs& r, uint8_t* dst, uint32_t sw) {
+    __device__ static __forceinline__ void emit_half(const Regs& r, uint32_t at) {
         const float d = __half2float(__ushort_as_half(static_cast<uint16_t>(r.d)));
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
@@ -427,7 +428,7 @@ struct GemmQ6KR {  // repacked groups of 224 B: scales[16] int8 | d fp16, pad | 
                     v[2 * k] = pack2<BF16>(mul2(ds2, widen(codes(bytes02(w), 32))));
                     v[2 * k + 1] = pack2<BF16>(mul2(ds2, widen(codes(bytes13(w), 32))));
                 }
-                store_chunk(dst, 4 * b + g, sw, make_uint4(v[0], v[1], v[2], v[3]));
+                store_chunk(at, 4 * b + g, make_uint4(v[0], v[1], v[2], v[3]));
             }
         }
     }
@@ -601,7 +602,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
         if (!ok && lane == 0) *abort_word = 1;
     } else if (warp >= kDeqWarp) {
         // ---- dequantization ----------------------------------------------------------------------------------------------------
-        const uint32_t j = (warp - kDeqWarp) / kDeqGroupWarps, r = ((warp - kDeqWarp) % kDeqGroupWarps) * 32u + lane, sw = r & 7u;
+        const uint32_t j = (warp - kDeqWarp) / kDeqGroupWarps, r = ((warp - kDeqWarp) % kDeqGroupWarps) * 32u + lane;
+        const uint32_t row_at = tiles + r * (kBK * 2u) + ((r & 7u) << 4);
         bool ok = true;
         RingPos rw{0, 0}, st{0, 0};
         st.advance(j, a.stages);
@@ -619,7 +621,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_const
                 rw.advance(1, a.raw_slots);
                 ok = g_mbar_wait_warp(empty(st.slot), st.parity ^ 1u);
                 if (!ok) break;
-                F::template emit<BF16>(regs, j, smem + st.slot * stage_bytes + r * (kBK * 2u), sw);
+                F::template emit<BF16>(regs, j, row_at + st.slot * stage_bytes);
                 // make the generic-proxy stores visible to the tensor core's (async-proxy) reads, then one arrival per warp
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
