@@ -26,6 +26,10 @@
 // weight) where it is small, HBM below that.  A pair shares the dequantized W: a CTA converts 128 rows for T tokens, and its quants arrive
 // by TMA instead of 16-byte gathers from 128 different rows.
 //
+// Measured against one 256 x 256 tile a CTA with gathered quants: Q4_K 17408 x 5120 at 512 / 2048 tokens 109 -> 74 / 393 -> 268 us
+// (1.36 PFLOP/s; 34816 x 5120 1.45, where the power cap holds the clock), Q6_K 5120 x 17408 at 2048 tokens 1070 -> 312 us, Q8_0 and Q4_0
+// 17408 x 5120 at 2048 tokens 262 us; at 64 tokens, Q4_0 / Q8_0 / Q4_K / Q6_K 17408 x 5120, 26 / 28 / 31 / 33 us.
+//
 // The K order inside every group of 8 elements is permuted to (0,2,1,3,4,6,5,7) in BOTH operands -- the cast kernel
 // writes X that way -- because that is the order in which masked nibble pairs fall out of a 32-bit word.
 //
@@ -806,17 +810,31 @@ cudaLaunchConfig_t dependent_launch(dim3 grid, uint32_t threads, uint32_t smem, 
     return cfg;
 }
 
+/// Scratch for the splits' partial sums, where it is there or can be had: a stream that is being captured cannot grow it (the growth waits
+/// for the stream), and a device without the memory need not, since the same plan runs with K unsplit.
+bool split_scratch(HaloCudaCtx* ctx, uint64_t bytes, cudaStream_t s, void** out) {
+    if (ctx->scratch[s].bytes[3] < bytes) {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    if (workspace(ctx, 3, bytes, s, out) == 0) return true;
+    cudaGetLastError();
+    return false;
+}
+
 template <bool BF16, class F>
 int launch_t(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
     const uint32_t pairs_max = static_cast<uint32_t>(ctx->prop.multiProcessorCount) / 2u;
-    const GemmPlan p = plan_gemm<F>(c.rows, c.cols, c.n_vec, pairs_max, (c.flags & HALO_CUDA_GEMV_FLAG_NO_SCRATCH) == 0);
-    const uint64_t rest = uint64_t{p.w_tiles} * p.token_tiles - p.whole;
-    if (p.units > 0x7FFFFFFFu) return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: %u x %u outputs exceed the launch limit", c.n_vec, c.rows);
+    GemmPlan p = plan_gemm<F>(c.rows, c.cols, c.n_vec, pairs_max, (c.flags & HALO_CUDA_GEMV_FLAG_NO_SCRATCH) == 0);
+    const uint64_t tiles = uint64_t{p.w_tiles} * p.token_tiles, rest = tiles - p.whole;
+    if (tiles > 0x7FFFFFFFu) return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: %u x %u outputs exceed the launch limit", c.n_vec, c.rows);
     void* ws = nullptr;
     if (int rc = workspace(ctx, 0, uint64_t{c.n_vec} * c.cols * 2, s, &ws)) return rc;
     void* partials = nullptr;
-    if (p.splits > 1)
-        if (int rc = workspace(ctx, 3, rest * p.splits * p.nacc * p.nt * kPairRows * 4u, s, &partials)) return rc;
+    if (p.splits > 1 && !split_scratch(ctx, rest * p.splits * p.nacc * p.nt * kPairRows * 4u, s, &partials)) p.splits = 1, p.whole = p.units = tiles;
     CUtensorMap xmap, wmap;
     if (int rc = encode_2d(BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, ws, c.cols, c.n_vec, uint64_t{c.cols} * 2, kBK, p.nt / 2u,
                            CU_TENSOR_MAP_SWIZZLE_128B, "x", &xmap))

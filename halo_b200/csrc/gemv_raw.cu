@@ -417,6 +417,7 @@ bool gemv_raw_supports(const GemvCall& c) {
 }
 
 int launch_gemv_raw(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
+    if (c.n_vec / 4 > 65535u) return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: n_vec %u exceeds the launch limit", c.n_vec);
     switch (c.wtype) {
         case HALO_CUDA_T_Q8_0: return launch_format<RawQ80>(ctx, c, s);
         case HALO_CUDA_T_Q4_0: return launch_format<RawQ40>(ctx, c, s);

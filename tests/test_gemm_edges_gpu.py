@@ -52,3 +52,43 @@ def test_gemm_tile_edges(be, checker, t, bf16, m, n, k):
     hw, hx = rounded(checker.dequantize(t, w, n * k).reshape(n, k), bf16), rounded(x, bf16)
     err = np.abs(got[0][:, :n].astype(np.float64) - hx @ hw.T)
     assert np.all(err <= (k + 4) * 2.0**-24 * (np.abs(hx) @ np.abs(hw).T))
+
+
+def test_gemm_split_scratch_is_not_grown_while_capturing(be, checker):
+    # hidden 2560 x 2048 at 77 tokens splits K on every device this runs on; a stream whose partial-sum scratch has never been grown
+    # captures the unsplit plan instead of failing
+    import torch
+    t, n, k, m = synth.Q4_K, 2560, 2048, 77
+    w, x = synth.quant_weights(t, n, k, 85, 1), synth.activations(m, k, 85, 2)
+    wb, xb = be.import_host_readonly(np.ascontiguousarray(w).view(np.uint8).reshape(-1)), be.import_host_readonly(x)
+    yb = be.allocate(m * n * 4)
+
+    def call(st, rows, cols):
+        be.gemv(st, hb.GemvArgs(t, hb.TensorRef.of(wb), hb.TensorRef.of(xb), hb.TensorRef.of(yb), rows, cols, m, capi.GEMM_TCGEN05_F16, allow_gemm=True))
+
+    def result(st):
+        y = np.empty((m, n), np.float32)
+        be.download(st, hb.TensorRef.of(yb), y)
+        st.wait()
+        return y
+
+    eager, captured = be.create_stream(), be.create_stream()
+    call(eager, n, k)
+    want = result(eager)
+    # the captured stream has its 16-bit copy of x (same size) from a call that does not split: one W tile of one row, unsplit by the flag
+    a = hb.GemvArgs(t, hb.TensorRef.of(wb), hb.TensorRef.of(xb), hb.TensorRef.of(yb), n, k, m, capi.GEMM_TCGEN05_F16, allow_gemm=True)
+    g = be._gemv_struct(a, "MATMUL", False)
+    g.flags |= capi.FLAG_NO_SCRATCH
+    import ctypes
+    assert be.lib.halo_cuda_gemv(be.ctx, ctypes.byref(g), captured.handle) == 0
+    captured.wait()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(captured.handle)):
+        call(captured, n, k)
+    be.upload(captured, hb.TensorRef.of(yb), np.full(m * n, -77.0, np.float32))
+    captured.wait()
+    graph.replay()
+    torch.cuda.synchronize()
+    got = result(captured)
+    hw, hx = rounded(checker.dequantize(t, w, n * k).reshape(n, k), False), rounded(x, False)
+    assert np.all(np.abs(got - want) <= 2 * (k + 4) * 2.0**-24 * (np.abs(hx) @ np.abs(hw).T))
