@@ -165,9 +165,9 @@ struct RowItem<HALO_CUDA_T_Q4_0> {
     __device__ static uint32_t at(int r) { return 16u * r; }
 };
 
-constexpr uint32_t kRowItems = 2;  // items a thread requests together
-
-template <uint32_t WT>
+/// kRowItems: items a thread requests together -- two where there are many, one where the time is a thread's own instructions (one row of
+/// 8192 Q6_K elements 2.41 us with two, 1.58 with one; 55 rows of 8192 Q8_0 elements 1.98 with two, 2.24 with one).
+template <uint32_t WT, uint32_t kRowItems>
 __global__ void __launch_bounds__(256) get_rows_wide_kernel(const uint8_t* __restrict__ table, uint64_t table_stride, const int32_t* __restrict__ ids,
                                                             float* __restrict__ out, uint64_t out_stride, uint32_t n_rows, uint32_t cols,
                                                             uint32_t* __restrict__ status) {
@@ -324,6 +324,8 @@ int launch_exact_t(const GemvCall& c, cudaStream_t s) {
     return 0;
 }
 
+constexpr uint64_t kManyRowItems = 148 * 256;  // eight warps of items an SM: where the two forms cross for all four formats
+
 /// The wide form where its loads and stores are aligned (any GGUF tensor in a dense table with 16-byte aligned output rows), the
 /// element form for everything else (F32 tables, odd addresses, unaligned outputs).
 template <uint32_t WT>
@@ -332,9 +334,14 @@ int launch_get_rows_t(const HaloCudaGetRows& a, uint64_t ts, uint64_t os, cudaSt
     if constexpr (WT != HALO_CUDA_T_F32) {
         using I = RowItem<WT>;
         if (reinterpret_cast<uintptr_t>(table) % I::kAlign == 0 && ts % I::kAlign == 0 && reinterpret_cast<uintptr_t>(a.out) % 16 == 0 && os % 16 == 0) {
-            const uint32_t items = a.cols / I::kBlockElems * I::kPerBlock, threads = items < 128u * kRowItems ? 64u : 256u;
-            get_rows_wide_kernel<WT><<<dim3((items + threads * kRowItems - 1) / (threads * kRowItems), a.n_ids), threads, 0, s>>>(
-                table, ts, a.ids, a.out, os, a.n_rows, a.cols, a.status);
+            const uint32_t items = a.cols / I::kBlockElems * I::kPerBlock;
+            if (uint64_t{items} * a.n_ids < kManyRowItems) {
+                get_rows_wide_kernel<WT, 1><<<dim3((items + 63u) / 64u, a.n_ids), 64, 0, s>>>(table, ts, a.ids, a.out, os, a.n_rows, a.cols, a.status);
+            } else {
+                const uint32_t threads = items < 256u ? 64u : 256u;
+                get_rows_wide_kernel<WT, 2><<<dim3((items + threads * 2u - 1) / (threads * 2u), a.n_ids), threads, 0, s>>>(
+                    table, ts, a.ids, a.out, os, a.n_rows, a.cols, a.status);
+            }
             HC_CUDA(cudaGetLastError());
             return 0;
         }

@@ -72,3 +72,21 @@ def test_repack_edges(be, t, groups, pad, offset):
         if t == synth.Q6_K:
             assert not np.any(out[:, :prb].reshape(rows, groups, 224)[..., 18:32])
         assert np.all(out[:, prb:] == 0x5A)
+
+
+@pytest.mark.parametrize("cols", (4864, 5120))  # a last pair of items that is half there, and whole ones
+@pytest.mark.parametrize("t", (synth.Q4_K, *REPACKABLE))
+def test_get_rows_many_ids(be, checker, t, cols):
+    rows, n = 5, 400  # enough items for the form with two a thread
+    w = synth.random_blocks_finite(t, rows, cols, 45, t)
+    ids = (np.arange(n, dtype=np.int32) * 3) % rows
+    st = be.create_stream()
+    tb, ib, ob, sb = be.import_host_readonly(w), be.import_host_readonly(ids), be.allocate(n * cols * 4), be.allocate(4)
+    be.get_rows(st, hb.GetRowsArgs(t, hb.TensorRef.of(tb), hb.TensorRef.of(ib), hb.TensorRef.of(ob), rows, cols, n), status=sb)
+    got, status = np.empty((n, cols), np.float32), np.empty(1, np.uint32)
+    be.download(st, hb.TensorRef.of(ob), got)
+    be.download(st, hb.TensorRef.of(sb), status)
+    st.wait()
+    assert status[0] == 0
+    want = np.stack([checker.dequantize(t, w[r], cols) for r in range(rows)])
+    assert np.array_equal(bits(got), bits(want[ids]))
