@@ -92,3 +92,29 @@ def test_gemm_split_scratch_is_not_grown_while_capturing(be, checker):
     got = result(captured)
     hw, hx = rounded(checker.dequantize(t, w, n * k).reshape(n, k), False), rounded(x, False)
     assert np.all(np.abs(got - want) <= 2 * (k + 4) * 2.0**-24 * (np.abs(hx) @ np.abs(hw).T))
+
+
+# Shapes whose cheapest tile takes both accumulators (320 to 448 tokens), with and without K splits, and ragged in rows and tokens; the
+# first and last W rows against the rounded operands.
+@pytest.mark.parametrize("t,n,k,m", [(synth.Q4_K, 3200, 13824, 259), (synth.Q6_K, 17895, 3328, 280), (synth.Q4_K, 16034, 3584, 282), (synth.Q6_K, 14222, 3840, 346),
+                                     (synth.Q4_0, 9461, 11008, 770)])
+def test_gemm_wide_tiles(be, checker, t, n, k, m):
+    st = be.create_stream()
+    block = synth.quant_weights(t, 640, k, 90 + m, 1)
+    rows = np.ascontiguousarray(block).view(np.uint8).reshape(640, -1)
+    w = np.ascontiguousarray(np.tile(rows, (-(-n // 640), 1))[:n])
+    x = synth.activations(m, k, 90 + m, 2)
+    wb, variant = be.import_host_readonly(w.reshape(-1)), capi.GEMM_TCGEN05_F16
+    if t != synth.Q4_K:
+        wb, variant = be.repack(st, t, hb.TensorRef.of(wb), n, k), capi.GEMM_TCGEN05_F16_R
+    xb, yb = be.import_host_readonly(x), be.allocate(m * n * 4)
+    be.gemv(st, hb.GemvArgs(t, hb.TensorRef.of(wb), hb.TensorRef.of(xb), hb.TensorRef.of(yb), n, k, m, variant, allow_gemm=True))
+    y = np.empty((m, n), np.float32)
+    be.download(st, hb.TensorRef.of(yb), y)
+    st.wait()
+    hw, hx = rounded(checker.dequantize(t, block, 640 * k).reshape(640, k), False), rounded(x, False)
+    ref, mag = hx @ hw.T, np.abs(hx) @ np.abs(hw).T
+    for first in range(0, n, 640):
+        r = min(640, n - first)
+        err = np.abs(y[:, first:first + r].astype(np.float64) - ref[:, :r])
+        assert np.all(err <= (k + 4) * 2.0**-24 * mag[:, :r]), f"rows from {first}"
