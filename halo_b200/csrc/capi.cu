@@ -66,21 +66,41 @@ int enter(HaloCudaCtx* ctx) {
     return 0;
 }
 
-int workspace(HaloCudaCtx* ctx, int slot, uint64_t bytes, cudaStream_t stream, void** out, bool zeroed) {
-    HaloCudaCtx::Scratch& sc = ctx->scratch[stream];  // the calling stream's own set: nothing another stream runs touches it
-    if (bytes > sc.bytes[slot]) {
-        // Work already enqueued on this stream may still read the old block: drain before releasing it.
-        HC_CUDA(cudaStreamSynchronize(stream));
-        if (sc.block[slot] != nullptr) HC_CUDA(cudaFree(sc.block[slot]));
-        sc.block[slot] = nullptr;
-        sc.bytes[slot] = 0;
-        const uint64_t want = (bytes + (1u << 20) - 1) & ~uint64_t{(1u << 20) - 1};
-        HC_CUDA(cudaMalloc(&sc.block[slot], want));
-        sc.bytes[slot] = want;
-        if (zeroed) HC_CUDA(cudaMemsetAsync(sc.block[slot], 0, want, stream));
+namespace {
+/// The calls a stream's scratch is made of (scratch.h).
+struct ScratchDriver {
+    cudaStream_t stream;
+    bool capturing() const {
+        if (stream == nullptr || stream == cudaStreamLegacy) return false;  // never captured, and asking about it disturbs a capture elsewhere
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        return cudaStreamIsCapturing(stream, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
     }
-    *out = sc.block[slot];
-    return 0;
+    int drain() const {
+        HC_CUDA(cudaStreamSynchronize(stream));
+        return 0;
+    }
+    int allocate(void** p, uint64_t bytes) const {
+        const cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaSuccess) return 0;
+        cudaGetLastError();
+        return fail(e == cudaErrorMemoryAllocation ? HALO_CUDA_E_MEMORY : HALO_CUDA_E_BACKEND, "cannot allocate %llu bytes of scratch: %s", (unsigned long long)bytes,
+                    cudaGetErrorString(e));
+    }
+    int release(void* p) const {
+        HC_CUDA(cudaFree(p));
+        return 0;
+    }
+    int clear(void* p, uint64_t bytes) const {
+        HC_CUDA(cudaMemsetAsync(p, 0, bytes, stream));
+        return 0;
+    }
+    int out_of_host_memory() const { return fail(HALO_CUDA_E_MEMORY, "out of host memory"); }
+};
+}  // namespace
+
+int workspace(HaloCudaCtx* ctx, int slot, uint64_t bytes, cudaStream_t stream, void** out, bool zeroed) {
+    ScratchDriver driver{stream};
+    return take_scratch(ctx->scratch[stream], slot, bytes, zeroed, driver, out);  // the calling stream's own set: nothing another stream runs touches it
 }
 
 bool reads_repacked_rows(uint32_t variant_id) {
@@ -360,9 +380,7 @@ int halo_cuda_ctx_destroy(HaloCudaCtx* ctx) {
             }
             cudaMemPoolDestroy(ctx->pool);
         }
-        for (auto& kv : ctx->scratch)
-            for (void* p : kv.second.block)
-                if (p != nullptr) cudaFree(p);
+        for (auto& kv : ctx->scratch) kv.second.each([](void* p) { cudaFree(p); });
         if (ctx->error_word_host != nullptr) cudaFreeHost(ctx->error_word_host);
         for (int i = 0; i < 2; ++i) {
             if (ctx->staging[i] != nullptr) cudaFreeHost(ctx->staging[i]);
@@ -476,8 +494,7 @@ int halo_cuda_stream_destroy(HaloCudaCtx* ctx, HaloCudaStream stream) {
     const auto it = ctx->scratch.find(s);
     if (it != ctx->scratch.end()) {  // the stream's scratch goes with it, once its work has drained
         cudaStreamSynchronize(s);
-        for (void* p : it->second.block)
-            if (p != nullptr) cudaFree(p);
+        it->second.each([](void* p) { cudaFree(p); });
         ctx->scratch.erase(it);
     }
     HC_CUDA(cudaStreamDestroy(s));
@@ -519,8 +536,7 @@ int halo_cuda_ctx_lost(HaloCudaCtx* ctx) { return ctx != nullptr && ctx->lost ? 
 int halo_cuda_ctx_scratch_bytes(HaloCudaCtx* ctx, uint64_t* bytes) {
     if (ctx == nullptr || bytes == nullptr) return fail(HALO_CUDA_E_API, "null argument");
     *bytes = 0;
-    for (const auto& kv : ctx->scratch)
-        for (uint64_t b : kv.second.bytes) *bytes += b;
+    for (const auto& kv : ctx->scratch) *bytes += kv.second.total();
     return 0;
 }
 

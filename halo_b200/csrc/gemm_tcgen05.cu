@@ -813,7 +813,7 @@ cudaLaunchConfig_t dependent_launch(dim3 grid, uint32_t threads, uint32_t smem, 
 /// Scratch for the splits' partial sums, where it is there or can be had: a stream that is being captured cannot grow it (the growth waits
 /// for the stream), and a device without the memory need not, since the same plan runs with K unsplit.
 bool split_scratch(HaloCudaCtx* ctx, uint64_t bytes, cudaStream_t s, void** out) {
-    if (ctx->scratch[s].bytes[3] < bytes) {
+    if (ctx->scratch[s].block[3].bytes < bytes) {
         cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) {
             cudaGetLastError();

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "halo_cuda.h"
+#include "scratch.h"
 
 namespace halo_cuda {
 
@@ -44,14 +45,7 @@ struct HaloCudaCtx {
     // Scratch for kernels that need global memory beyond their operands (activation staging, split-K
     // partials).  Grown on demand and reused in stream order, so every stream has a set of its own: calls on different
     // streams of one context may overlap on the device without sharing counters, partials or staged x.  One thread drives a context.
-    // Slot 0 serves the matmul kernels, slot 1 the LM head (its logits and argmax partials live across a matmul),
-    // slot 2 the row-block counters of the balanced kernels (zeroed when allocated, left zeroed by every kernel),
-    // slot 3 their partial sums.
-    struct Scratch {
-        void* block[4] = {nullptr, nullptr, nullptr, nullptr};
-        uint64_t bytes[4] = {0, 0, 0, 0};
-    };
-    std::unordered_map<cudaStream_t, Scratch> scratch;
+    std::unordered_map<cudaStream_t, halo_cuda::Scratch> scratch;
     std::vector<halo_cuda::PlanEntry> plan;
     // One word of mapped pinned host memory that kernels OR error bits into (bit 0: a bounded device-side wait
     // expired).  The host reads it after every stream wait; a set bit marks the context lost.
@@ -80,8 +74,8 @@ namespace halo_cuda {
 
 /// Makes ctx's device current; E_API for a null ctx, E_DEVICE once the context is lost.
 int enter(HaloCudaCtx* ctx);
-/// Returns ctx scratch of at least `bytes` (grows with cudaMalloc; earlier contents are dropped; `zeroed` clears a
-/// newly allocated block in stream order).
+/// Returns ctx scratch of at least `bytes` (grows with cudaMalloc by the rule of take_scratch; earlier contents are dropped; `zeroed`
+/// clears a newly allocated block in stream order).
 int workspace(HaloCudaCtx* ctx, int slot, uint64_t bytes, cudaStream_t stream, void** out, bool zeroed = false);
 /// Raises the dynamic shared-memory limit of `kernel` to `bytes` on ctx's device, once per context.
 int allow_dynamic_smem(HaloCudaCtx* ctx, const void* kernel, uint32_t bytes);

@@ -174,6 +174,8 @@ int halo_cuda_ctx_lost(HaloCudaCtx* ctx); /* 1 once a wait timed out or the devi
 int halo_cuda_ctx_set_peer_wait_polls(HaloCudaCtx* ctx, uint32_t polls);
 /* Streams and scratch: the kernels' on-demand scratch is kept per stream, so calls on different streams of one context may overlap on
  * the device; calls on ONE stream reuse that stream's scratch in stream order.  halo_cuda_stream_destroy releases the stream's scratch.
+ * A call captured into a CUDA graph holds the address of its stream's scratch: that block stays until the stream or the context is
+ * destroyed, also when later calls grow the scratch, so the graph may be replayed (in order with the stream's other work) until then.
  * (halo_cuda_lm_head_noalloc is the exception: its fixed array is shared by every call on the GPU.)
  * Bytes of context scratch (staged activations, split-K partials, LM-head logits and argmax partials) the context holds right now:
  * memory the kernels allocated on demand beyond the caller's operands.  Stays 0 for a context that only ever made calls that need

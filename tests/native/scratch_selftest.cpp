@@ -1,0 +1,71 @@
+// The growth rule of a stream's scratch (halo_b200/csrc/scratch.h) against a driver that keeps books instead of allocating.
+#include <cstdio>
+#include <cstdlib>
+#include <set>
+
+#include "scratch.h"
+
+using namespace halo_cuda;
+
+#define CHECK(cond)                                                             \
+    do {                                                                        \
+        if (!(cond)) std::printf("line %d: %s\n", __LINE__, #cond), std::exit(1); \
+    } while (0)
+
+constexpr uint64_t MB = 1u << 20;
+constexpr int kNoMemory = -2, kRefused = -3;
+
+struct Books {
+    bool in_capture = false;
+    uint64_t limit = UINT64_MAX;  // an allocation above it fails
+    std::set<void*> live;
+    int drains = 0, clears = 0;
+    uintptr_t next = 0x1000;
+
+    bool capturing() const { return in_capture; }
+    int drain() { return in_capture ? kRefused : (++drains, 0); }
+    int allocate(void** p, uint64_t bytes) {
+        if (bytes > limit) return kNoMemory;
+        live.insert(*p = reinterpret_cast<void*>(next++));
+        return 0;
+    }
+    int release(void* p) {
+        CHECK(live.erase(p) == 1);
+        return 0;
+    }
+    int clear(void*, uint64_t) { return ++clears, 0; }
+    int out_of_host_memory() const { return kNoMemory; }
+};
+
+int main() {
+    Books d;
+    Scratch s;
+    void *a = nullptr, *b = nullptr, *c = nullptr;
+    // eager calls: one block, released when a larger one replaces it
+    CHECK(take_scratch(s, 3, 1, false, d, &a) == 0 && s.block[3].bytes == MB && d.live.count(a));
+    CHECK(take_scratch(s, 3, MB, false, d, &b) == 0 && b == a);
+    CHECK(take_scratch(s, 3, MB + 1, false, d, &b) == 0 && b != a && !d.live.count(a) && s.block[3].bytes == 2 * MB && s.kept.empty());
+    // a graph takes the block's address: growth keeps the block, and at least doubles
+    d.in_capture = true;
+    CHECK(take_scratch(s, 3, 5, false, d, &a) == 0 && a == b);
+    CHECK(take_scratch(s, 3, 3 * MB, false, d, &c) == kRefused && d.live.count(a) && s.block[3].p == a);  // never grown while capturing
+    d.in_capture = false;
+    CHECK(take_scratch(s, 3, 2 * MB + 1, false, d, &c) == 0 && c != a && d.live.count(a) && s.block[3].bytes == 4 * MB);
+    CHECK(s.kept.size() == 1 && s.kept[0].p == a && s.total() == 6 * MB);
+    // the new block is in no graph: it goes when it is outgrown
+    CHECK(take_scratch(s, 3, 9 * MB, false, d, &b) == 0 && !d.live.count(c) && d.live.count(a) && s.block[3].bytes == 9 * MB);
+    // another slot of the stream is its own; one that is cleared is cleared whenever it is new
+    CHECK(take_scratch(s, 2, 8, true, d, &c) == 0 && d.clears == 1 && take_scratch(s, 2, 8, true, d, &c) == 0 && d.clears == 1);
+    d.in_capture = true;
+    CHECK(take_scratch(s, 2, 8, true, d, &a) == 0 && a == c && take_scratch(s, 3, MB, false, d, &a) == 0 && a == b);
+    d.in_capture = false;
+    CHECK(take_scratch(s, 2, 2 * MB, true, d, &a) == 0 && d.clears == 2 && d.live.count(c));
+    // a graph's slot grows by what is needed where twice as much is not to be had, and a refused growth leaves the graph's block alive
+    d.limit = 10 * MB;
+    CHECK(take_scratch(s, 3, 10 * MB, false, d, &a) == 0 && s.block[3].bytes == 10 * MB && d.live.count(b));
+    CHECK(take_scratch(s, 3, 11 * MB, false, d, &a) == kNoMemory && d.live.count(b) && s.block[3].p == nullptr && s.block[3].bytes == 0);
+    CHECK(take_scratch(s, 3, MB, false, d, &a) == 0 && s.block[3].bytes == MB);
+    s.each([&](void* p) { d.release(p); });
+    CHECK(d.live.empty());
+    return 0;
+}
