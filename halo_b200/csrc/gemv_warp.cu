@@ -1,5 +1,5 @@
 // gemv_warp_f32: the fp32 CUDA-core streaming kernel for decode-shaped calls, all four block formats.  Q4_K rows, and raw rows of the
-// other formats whose K is too long for gemv_raw.cu's shared memory, run the kernel below; the rest runs there.
+// other formats whose K is too long for gemv_raw.cu's shared memory or too short for its warps, run the kernel below; the rest runs there.
 //
 // One warp owns one W row.  The row is cut into 16- or 32-weight chunks; lane L takes chunks L, L+32, ... so a
 // warp-wide load walks the row front to back in runs of whole sectors.  Inside a chunk the sub-block scale is

@@ -117,7 +117,7 @@ __device__ __forceinline__ float gated_value(float y, uint32_t n, uint32_t n_v, 
 // kernel launchers (one per translation unit); each returns a status
 int launch_gemv_exact8(const GemvCall& c, cudaStream_t s);
 int launch_gemv_warp_f32(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s);
-bool gemv_raw_supports(const GemvCall& c);  // raw Q8_0 / Q4_0 / Q6_K rows whose x fits in shared memory: gemv_warp_f32 through gemv_raw.cu
+bool gemv_raw_supports(const GemvCall& c);  // raw Q8_0 / Q4_0 / Q6_K rows whose x fits in shared memory and whose K is not too short: gemv_warp_f32 through gemv_raw.cu
 int launch_gemv_raw(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s);
 bool gemv_warp_f32_supports(const GemvCall& c);
 int launch_gemv_mma(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s);

@@ -1,5 +1,6 @@
 """gemv_warp_f32 over raw Q8_0 / Q4_0 / Q6_K rows at the edges of its shared-memory form: K around a lane's 64 weights and a slot's 2048,
-rows around a warp's passes, every batch form, rows at any even address, and a K just beyond what fits (the form without shared memory).
+rows around a warp's passes, every batch form, rows at any even address, the shortest K each format takes and the longest below it, and a K
+just beyond what fits (both: the form without shared memory).
 
 Bounds: against the fp64 product of the exact weights, each product, group sum, group term and tree level rounds once, at most
 (K / 32 + 32 + 8) roundings of 2^-24 on sum |w x|."""
@@ -33,7 +34,7 @@ def run(be, st, t, wb, offset, stride, x, n, k):
 
 
 @pytest.mark.parametrize("t", (synth.Q8_0, synth.Q4_0, synth.Q6_K))
-@pytest.mark.parametrize("n,k", [(1, 32), (7, 96), (37, 2048), (300, 2080), (95, 5120), (1185, 288), (33, 8192), (24, 17408), (9, 28672), (3, 65536)])
+@pytest.mark.parametrize("n,k", [(1, 32), (7, 96), (37, 2048), (300, 2080), (95, 5120), (1185, 288), (70, 352), (70, 384), (41, 608), (41, 640), (50, 1024), (50, 1280), (33, 8192), (24, 17408), (9, 28672), (3, 65536)])
 @pytest.mark.parametrize("pad,offset", ((0, 0), (6, 2), (2, 14)))
 def test_raw_rows_edges(be, checker, t, n, k, pad, offset):
     k = -(-k // synth.BLOCK_ELEMS[t]) * synth.BLOCK_ELEMS[t]
