@@ -205,9 +205,13 @@ int launch_gemv_mma_r(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
 int launch_repack(uint32_t wtype, const void* src, uint64_t src_stride, void* dst, uint64_t dst_stride, uint32_t rows, uint32_t cols, cudaStream_t s) {
     const uint32_t groups = cols / 256u, words = group_bytes(wtype) / 4u;
     const uint8_t* from = static_cast<const uint8_t*>(src);
-    // Two-byte aligned rows (every GGUF tensor) take the tiled form, rows at odd addresses the word-by-word one.
-    if (reinterpret_cast<uintptr_t>(from) % 2 == 0 && src_stride % 2 == 0 && groups != 0) {
-        uint8_t* to = static_cast<uint8_t*>(dst);
+    uint8_t* to = static_cast<uint8_t*>(dst);
+    // Two-byte aligned rows (every GGUF tensor) take the tiled form, rows at odd addresses the word-by-word one -- and so do short rows of a
+    // strided matrix, of which a tile holds one each: 151936 rows of one / two / four Q4_0 groups 26 / 50 / 100 us by words and 114 / 151 / 175
+    // by tiles, of eight 197 and 183; Q8_0 and Q6_K cross between three and five groups, all three at about a kilobyte a row.
+    const uint64_t raw_row = uint64_t{groups} * (wtype == HALO_CUDA_T_Q4_0 ? 144u : wtype == HALO_CUDA_T_Q8_0 ? 272u : 210u);
+    const bool dense = src_stride == raw_row && dst_stride == uint64_t{groups} * words * 4u;
+    if (reinterpret_cast<uintptr_t>(from) % 2 == 0 && src_stride % 2 == 0 && groups != 0 && (dense || rows == 1 || raw_row >= 1024u)) {
         switch (wtype) {
             case HALO_CUDA_T_Q4_0: return launch_repack_tiled<HALO_CUDA_T_Q4_0>(from, src_stride, to, dst_stride, rows, groups, s);
             case HALO_CUDA_T_Q8_0: return launch_repack_tiled<HALO_CUDA_T_Q8_0>(from, src_stride, to, dst_stride, rows, groups, s);
