@@ -53,6 +53,12 @@ class GemvTiles(C.Structure):
                 ("stretch_cols", C.c_uint32), ("resident_rows", C.c_uint32), ("reserved", C.c_uint32 * 2)]
 
 
+class GemmPlan(C.Structure):
+    _fields_ = [("tile_tokens", C.c_uint32), ("accumulators", C.c_uint32), ("stages", C.c_uint32), ("raw_slots", C.c_uint32),
+                ("row_tiles", C.c_uint32), ("token_tiles", C.c_uint32), ("splits", C.c_uint32), ("pairs", C.c_uint32),
+                ("whole", C.c_uint64), ("units", C.c_uint64)]
+
+
 class PeerReduce(C.Structure):
     _fields_ = [("world", C.c_uint32), ("rank", C.c_uint32), ("capacity", C.c_uint32), ("reserved", C.c_uint32),
                 ("slots", C.c_void_p * 8), ("epoch", C.c_void_p), ("done", C.c_void_p)]
@@ -127,6 +133,7 @@ SYMBOLS = {
     "halo_cuda_repacked_row_bytes": (C.c_int, [C.c_uint32, C.c_uint64, C.POINTER(C.c_uint64)]),
     "halo_cuda_gemv_plan_i8": (C.c_int, [C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.POINTER(GemvPlan)]),
     "halo_cuda_gemv_tiles_i8": (C.c_int, [C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.POINTER(GemvTiles)]),
+    "halo_cuda_gemm_plan": (C.c_int, [C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.POINTER(GemmPlan)]),
     "halo_cuda_repacked_variant": (C.c_int, [C.c_uint32, C.c_uint64, C.POINTER(C.c_uint32)]),
     "halo_cuda_repack_rows": (C.c_int, [_P, C.c_uint32, _P, C.c_uint64, _P, C.c_uint64, C.c_uint32, C.c_uint32, _P]),
     "halo_cuda_gemv_plan": (C.c_int, [C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.POINTER(GemvPlan)]),

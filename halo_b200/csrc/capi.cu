@@ -80,7 +80,12 @@ struct ScratchDriver {
         return 0;
     }
     int allocate(void** p, uint64_t bytes) const {
+        // Any thread's capture forbids an allocation in the default mode, which is there for calls whose order against the captured work is in
+        // doubt; a fresh block has none.
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        const bool relaxed = capturing() && cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
         const cudaError_t e = cudaMalloc(p, bytes);
+        if (relaxed) cudaThreadExchangeStreamCaptureMode(&mode);
         if (e == cudaSuccess) return 0;
         cudaGetLastError();
         return fail(e == cudaErrorMemoryAllocation ? HALO_CUDA_E_MEMORY : HALO_CUDA_E_BACKEND, "cannot allocate %llu bytes of scratch: %s", (unsigned long long)bytes,
@@ -98,9 +103,9 @@ struct ScratchDriver {
 };
 }  // namespace
 
-int workspace(HaloCudaCtx* ctx, int slot, uint64_t bytes, cudaStream_t stream, void** out, bool zeroed) {
+int workspace(HaloCudaCtx* ctx, int slot, uint64_t bytes, cudaStream_t stream, void** out, bool zeroed, bool while_capturing) {
     ScratchDriver driver{stream};
-    return take_scratch(ctx->scratch[stream], slot, bytes, zeroed, driver, out);  // the calling stream's own set: nothing another stream runs touches it
+    return take_scratch(ctx->scratch[stream], slot, bytes, zeroed, while_capturing, driver, out);  // the calling stream's own set: nothing another stream runs touches it
 }
 
 bool reads_repacked_rows(uint32_t variant_id) {
@@ -816,6 +821,13 @@ int halo_cuda_gemv_tiles_i8(uint32_t wtype, uint32_t rows, uint32_t cols, uint32
     }
     if (tiles->resident_rows == 0) return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: the int8 kernels keep x in shared memory; %u columns do not fit", cols);
     return 0;
+}
+
+int halo_cuda_gemm_plan(uint32_t wtype, uint32_t rows, uint32_t cols, uint32_t n_vec, uint32_t sm_count, uint32_t flags, HaloCudaGemmPlan* plan) {
+    if (plan == nullptr) return fail(HALO_CUDA_E_API, "null argument");
+    if (cols == 0 || cols % 256u != 0) return fail(HALO_CUDA_E_MODEL, "MATMUL: %u elements is not a multiple of 256", cols);
+    if (rows == 0 || n_vec == 0 || sm_count < 2u) return fail(HALO_CUDA_E_KERNEL, "MATMUL: empty matrix, or a device without a pair of SMs");
+    return gemm_plan(wtype, rows, cols, n_vec, sm_count, (flags & HALO_CUDA_GEMV_FLAG_NO_SCRATCH) == 0, plan);
 }
 
 int halo_cuda_gemv_reduce(HaloCudaCtx* ctx, const HaloCudaGemv* args, const HaloCudaPeerReduce* peers, HaloCudaStream stream) {

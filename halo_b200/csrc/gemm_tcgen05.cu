@@ -758,6 +758,7 @@ int encode_2d(CUtensorMapDataType type, const void* base, uint64_t inner, uint64
 struct GemmPlan {
     uint32_t nt, nacc, stages, raw_slots, w_tiles, token_tiles, splits;
     uint64_t whole, units;  // tiles over all of K; units of work
+    uint64_t split_tiles() const { return uint64_t{w_tiles} * token_tiles - whole; }
 };
 
 template <class F>
@@ -810,31 +811,21 @@ cudaLaunchConfig_t dependent_launch(dim3 grid, uint32_t threads, uint32_t smem, 
     return cfg;
 }
 
-/// Scratch for the splits' partial sums, where it is there or can be had: a stream that is being captured cannot grow it (the growth waits
-/// for the stream), and a device without the memory need not, since the same plan runs with K unsplit.
-bool split_scratch(HaloCudaCtx* ctx, uint64_t bytes, cudaStream_t s, void** out) {
-    if (ctx->scratch[s].block[3].bytes < bytes) {
-        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-            return false;
-        }
-    }
-    if (workspace(ctx, 3, bytes, s, out) == 0) return true;
-    cudaGetLastError();
-    return false;
-}
-
 template <bool BF16, class F>
 int launch_t(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
     const uint32_t pairs_max = static_cast<uint32_t>(ctx->prop.multiProcessorCount) / 2u;
     GemmPlan p = plan_gemm<F>(c.rows, c.cols, c.n_vec, pairs_max, (c.flags & HALO_CUDA_GEMV_FLAG_NO_SCRATCH) == 0);
-    const uint64_t tiles = uint64_t{p.w_tiles} * p.token_tiles, rest = tiles - p.whole;
-    if (tiles > 0x7FFFFFFFu) return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: %u x %u outputs exceed the launch limit", c.n_vec, c.rows);
+    if (uint64_t{p.w_tiles} * p.token_tiles > 0x7FFFFFFFu) return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: %u x %u outputs exceed the launch limit", c.n_vec, c.rows);
     void* ws = nullptr;
     if (int rc = workspace(ctx, 0, uint64_t{c.n_vec} * c.cols * 2, s, &ws)) return rc;
+    // The splits' partial sums: also while the stream is being captured, so that a prompt's plan, and with it its bits, do not depend on what the
+    // stream ran before.  A device without the memory runs the cheapest plan that needs none.
     void* partials = nullptr;
-    if (p.splits > 1 && !split_scratch(ctx, rest * p.splits * p.nacc * p.nt * kPairRows * 4u, s, &partials)) p.splits = 1, p.whole = p.units = tiles;
+    if (p.splits > 1) {
+        const int rc = workspace(ctx, 4, p.split_tiles() * p.splits * p.nacc * p.nt * kPairRows * 4u, s, &partials, /*zeroed=*/false, /*while_capturing=*/true);
+        if (rc == HALO_CUDA_E_MEMORY) p = plan_gemm<F>(c.rows, c.cols, c.n_vec, pairs_max, false);
+        else if (rc != 0) return rc;
+    }
     CUtensorMap xmap, wmap;
     if (int rc = encode_2d(BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, ws, c.cols, c.n_vec, uint64_t{c.cols} * 2, kBK, p.nt / 2u,
                            CU_TENSOR_MAP_SWIZZLE_128B, "x", &xmap))
@@ -854,7 +845,7 @@ int launch_t(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
     const cudaLaunchConfig_t cfg = dependent_launch(dim3(2u * static_cast<uint32_t>(std::min<uint64_t>(p.units, pairs_max))), kGemmThreads, kGemmSmem, s, attr);
     HC_CUDA(cudaLaunchKernelEx(&cfg, kern, xmap, wmap, args));
     if (p.splits > 1) {
-        const cudaLaunchConfig_t add_cfg = dependent_launch(dim3(2u * static_cast<uint32_t>(rest), p.nacc * p.nt / 8u), 128, 0, s, attr);
+        const cudaLaunchConfig_t add_cfg = dependent_launch(dim3(2u * static_cast<uint32_t>(p.split_tiles()), p.nacc * p.nt / 8u), 128, 0, s, attr);
         HC_CUDA(cudaLaunchKernelEx(&add_cfg, add_splits_kernel, static_cast<const float*>(partials), c.y, c.y_stride, c.rows, c.n_vec, p.nacc * p.nt, p.token_tiles, static_cast<uint32_t>(p.whole), p.splits));
     }
     return 0;
@@ -883,6 +874,20 @@ int launch_gemm_tcgen05(HaloCudaCtx* ctx, const GemvCall& c, bool bf16, bool rep
         case HALO_CUDA_T_Q8_0: return launch_f<GemmQ80R>(ctx, c, bf16, s);
         case HALO_CUDA_T_Q4_0: return launch_f<GemmQ40R>(ctx, c, bf16, s);
         default: return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: no repacked GEMM for weight type id %u", c.wtype);
+    }
+}
+
+int gemm_plan(uint32_t wtype, uint32_t rows, uint32_t cols, uint32_t n_vec, uint32_t sm_count, bool may_split, HaloCudaGemmPlan* out) {
+    auto describe = [&](const GemmPlan& p) {
+        *out = HaloCudaGemmPlan{p.nt * p.nacc, p.nacc, p.stages, p.raw_slots, p.w_tiles, p.token_tiles, p.splits, sm_count / 2u, p.whole, p.units};
+        return 0;
+    };
+    switch (wtype) {
+        case HALO_CUDA_T_Q4_K: return describe(plan_gemm<GemmQ4K>(rows, cols, n_vec, sm_count / 2u, may_split));
+        case HALO_CUDA_T_Q6_K: return describe(plan_gemm<GemmQ6KR>(rows, cols, n_vec, sm_count / 2u, may_split));
+        case HALO_CUDA_T_Q8_0: return describe(plan_gemm<GemmQ80R>(rows, cols, n_vec, sm_count / 2u, may_split));
+        case HALO_CUDA_T_Q4_0: return describe(plan_gemm<GemmQ40R>(rows, cols, n_vec, sm_count / 2u, may_split));
+        default: return fail(HALO_CUDA_E_UNSUPPORTED, "MATMUL: no prefill GEMM for weight type id %u", wtype);
     }
 }
 

@@ -75,8 +75,8 @@ namespace halo_cuda {
 /// Makes ctx's device current; E_API for a null ctx, E_DEVICE once the context is lost.
 int enter(HaloCudaCtx* ctx);
 /// Returns ctx scratch of at least `bytes` (grows with cudaMalloc by the rule of take_scratch; earlier contents are dropped; `zeroed`
-/// clears a newly allocated block in stream order).
-int workspace(HaloCudaCtx* ctx, int slot, uint64_t bytes, cudaStream_t stream, void** out, bool zeroed = false);
+/// clears a newly allocated block in stream order; `while_capturing`: grows while the stream is being captured, too).
+int workspace(HaloCudaCtx* ctx, int slot, uint64_t bytes, cudaStream_t stream, void** out, bool zeroed = false, bool while_capturing = false);
 /// Raises the dynamic shared-memory limit of `kernel` to `bytes` on ctx's device, once per context.
 int allow_dynamic_smem(HaloCudaCtx* ctx, const void* kernel, uint32_t bytes);
 /// The bookkeeping of allow_dynamic_smem without the driver call: true when (ctx, kernel) was not yet recorded.
@@ -162,6 +162,7 @@ bool gemv_mma_r_supports(const GemvCall& c);
 uint64_t repacked_row_bytes(uint32_t wtype, uint64_t cols);  // 0 for a type without a repacked layout
 int launch_repack(uint32_t wtype, const void* src, uint64_t src_stride, void* dst, uint64_t dst_stride, uint32_t rows, uint32_t cols, cudaStream_t s);
 bool gemm_tcgen05_supports(const GemvCall& c, bool repacked = false);
+int gemm_plan(uint32_t wtype, uint32_t rows, uint32_t cols, uint32_t n_vec, uint32_t sm_count, bool may_split, HaloCudaGemmPlan* out);
 int launch_get_rows(const HaloCudaGetRows& a, uint64_t row_bytes, uint64_t table_stride, uint64_t out_stride, cudaStream_t s);
 int launch_argmax(const float* logits, uint64_t stride_elems, uint32_t n, uint32_t n_vec, uint32_t valid, uint32_t row_offset,
                   uint32_t* result, int32_t* ids, void* scratch, cudaStream_t s);

@@ -14,9 +14,10 @@ struct ScratchBlock {
 };
 
 /// Slot 0 serves the matmul kernels (staged x), slot 1 the LM head (its logits and argmax partials live across a matmul), slot 2 the row-block
-/// counters of the balanced kernels (zeroed when allocated, left zeroed by every kernel), slot 3 their partial sums.
+/// counters of the balanced kernels (zeroed when allocated, left zeroed by every kernel), slot 3 their partial sums, slot 4 the partial sums of
+/// the prefill GEMM's K splits (its own, so that a prompt that cannot have them leaves what a decode step needs).
 struct Scratch {
-    static constexpr int kSlots = 4;
+    static constexpr int kSlots = 5;
     ScratchBlock block[kSlots];
     std::vector<ScratchBlock> kept;  // outgrown blocks whose address a graph holds: they live as long as the stream's scratch
 
@@ -36,17 +37,19 @@ struct Scratch {
 
 /// A block of at least `bytes` in `slot`.  A larger request replaces the block; its contents are dropped.  The old block is released once the
 /// stream has drained, unless a graph holds its address: then it is kept, and the new one is at least twice its size, so that what a slot keeps
-/// stays below what it holds.  Driver: capturing(), drain(), allocate(&p, bytes), release(p), clear(p, bytes), out_of_memory(status).
+/// stays below what it holds.  A stream that is being captured cannot be waited for: `while_capturing` says that the slot grows there too (the
+/// old block is kept then), else the request is refused.
+/// Driver: capturing(), drain(), allocate(&p, bytes), release(p), clear(p, bytes), out_of_host_memory().
 template <class Driver>
-int take_scratch(Scratch& set, int slot, uint64_t bytes, bool zeroed, Driver& driver, void** out) {
+int take_scratch(Scratch& set, int slot, uint64_t bytes, bool zeroed, bool while_capturing, Driver& driver, void** out) {
     constexpr uint64_t kUnit = 1u << 20;
     ScratchBlock& b = set.block[slot];
     if (bytes > b.bytes) {
         uint64_t want = (bytes + kUnit - 1) & ~(kUnit - 1), least = want;
-        // Work already enqueued on this stream may still read the old block.  (A stream that is being captured cannot be waited for: it refuses.)
-        if (!b.in_graph || driver.capturing())
+        const bool capturing = driver.capturing(), keep = b.p != nullptr && (b.in_graph || (capturing && while_capturing));
+        if (capturing ? !while_capturing : !keep)  // work already enqueued on this stream may still read the old block
             if (int rc = driver.drain()) return rc;
-        if (b.in_graph) {
+        if (keep) {
             try {
                 set.kept.push_back(b);
             } catch (const std::bad_alloc&) {

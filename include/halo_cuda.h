@@ -253,6 +253,20 @@ typedef struct HaloCudaGemvTiles {
     uint32_t reserved[2];
 } HaloCudaGemvTiles;
 int halo_cuda_gemv_tiles_i8(uint32_t wtype, uint32_t rows, uint32_t cols, uint32_t n_vec, uint32_t sm_count, HaloCudaGemvTiles* tiles);
+/* How the prefill GEMM (variants 4, 5, 10, 11) cuts a call (host arithmetic, like the plans above): tiles of 256 W rows x `tile_tokens` x
+ * rows, dealt to `pairs` CTA pairs.  Tiles [0, whole) run over all of K; K of every tile behind them is cut into `splits` shares, whose sums
+ * are added in order: the order in which a row is added up depends on the shape and n_vec, and on nothing else.  With
+ * HALO_CUDA_GEMV_FLAG_NO_SCRATCH in `flags` the cheapest plan without splits (whole == tiles, splits == 1), which is also what a call runs
+ * that cannot have the memory for its splits' sums. */
+typedef struct HaloCudaGemmPlan {
+    uint32_t tile_tokens;   /* 32 to 448 */
+    uint32_t accumulators;  /* 1 (up to 256 tokens: a tile's results are stored under the next tile's products) or 2 */
+    uint32_t stages, raw_slots; /* rings of operand tiles and of quantized blocks in shared memory */
+    uint32_t row_tiles, token_tiles;
+    uint32_t splits, pairs;
+    uint64_t whole, units;  /* units = whole + (row_tiles * token_tiles - whole) * splits */
+} HaloCudaGemmPlan;
+int halo_cuda_gemm_plan(uint32_t wtype, uint32_t rows, uint32_t cols, uint32_t n_vec, uint32_t sm_count, uint32_t flags, HaloCudaGemmPlan* plan);
 
 /* ---- the operators ------------------------------------------------------------------------------ */
 int halo_cuda_gemv(HaloCudaCtx* ctx, const HaloCudaGemv* args, HaloCudaStream stream);

@@ -42,29 +42,43 @@ int main() {
     Scratch s;
     void *a = nullptr, *b = nullptr, *c = nullptr;
     // eager calls: one block, released when a larger one replaces it
-    CHECK(take_scratch(s, 3, 1, false, d, &a) == 0 && s.block[3].bytes == MB && d.live.count(a));
-    CHECK(take_scratch(s, 3, MB, false, d, &b) == 0 && b == a);
-    CHECK(take_scratch(s, 3, MB + 1, false, d, &b) == 0 && b != a && !d.live.count(a) && s.block[3].bytes == 2 * MB && s.kept.empty());
+    CHECK(take_scratch(s, 3, 1, false, false, d, &a) == 0 && s.block[3].bytes == MB && d.live.count(a));
+    CHECK(take_scratch(s, 3, MB, false, false, d, &b) == 0 && b == a);
+    CHECK(take_scratch(s, 3, MB + 1, false, false, d, &b) == 0 && b != a && !d.live.count(a) && s.block[3].bytes == 2 * MB && s.kept.empty());
     // a graph takes the block's address: growth keeps the block, and at least doubles
     d.in_capture = true;
-    CHECK(take_scratch(s, 3, 5, false, d, &a) == 0 && a == b);
-    CHECK(take_scratch(s, 3, 3 * MB, false, d, &c) == kRefused && d.live.count(a) && s.block[3].p == a);  // never grown while capturing
+    CHECK(take_scratch(s, 3, 5, false, false, d, &a) == 0 && a == b);
+    CHECK(take_scratch(s, 3, 3 * MB, false, false, d, &c) == kRefused && d.live.count(a) && s.block[3].p == a);  // never grown while capturing
     d.in_capture = false;
-    CHECK(take_scratch(s, 3, 2 * MB + 1, false, d, &c) == 0 && c != a && d.live.count(a) && s.block[3].bytes == 4 * MB);
+    CHECK(take_scratch(s, 3, 2 * MB + 1, false, false, d, &c) == 0 && c != a && d.live.count(a) && s.block[3].bytes == 4 * MB);
     CHECK(s.kept.size() == 1 && s.kept[0].p == a && s.total() == 6 * MB);
     // the new block is in no graph: it goes when it is outgrown
-    CHECK(take_scratch(s, 3, 9 * MB, false, d, &b) == 0 && !d.live.count(c) && d.live.count(a) && s.block[3].bytes == 9 * MB);
+    CHECK(take_scratch(s, 3, 9 * MB, false, false, d, &b) == 0 && !d.live.count(c) && d.live.count(a) && s.block[3].bytes == 9 * MB);
     // another slot of the stream is its own; one that is cleared is cleared whenever it is new
-    CHECK(take_scratch(s, 2, 8, true, d, &c) == 0 && d.clears == 1 && take_scratch(s, 2, 8, true, d, &c) == 0 && d.clears == 1);
+    CHECK(take_scratch(s, 2, 8, true, false, d, &c) == 0 && d.clears == 1 && take_scratch(s, 2, 8, true, false, d, &c) == 0 && d.clears == 1);
     d.in_capture = true;
-    CHECK(take_scratch(s, 2, 8, true, d, &a) == 0 && a == c && take_scratch(s, 3, MB, false, d, &a) == 0 && a == b);
+    CHECK(take_scratch(s, 2, 8, true, false, d, &a) == 0 && a == c && take_scratch(s, 3, MB, false, false, d, &a) == 0 && a == b);
     d.in_capture = false;
-    CHECK(take_scratch(s, 2, 2 * MB, true, d, &a) == 0 && d.clears == 2 && d.live.count(c));
+    CHECK(take_scratch(s, 2, 2 * MB, true, false, d, &a) == 0 && d.clears == 2 && d.live.count(c));
     // a graph's slot grows by what is needed where twice as much is not to be had, and a refused growth leaves the graph's block alive
     d.limit = 10 * MB;
-    CHECK(take_scratch(s, 3, 10 * MB, false, d, &a) == 0 && s.block[3].bytes == 10 * MB && d.live.count(b));
-    CHECK(take_scratch(s, 3, 11 * MB, false, d, &a) == kNoMemory && d.live.count(b) && s.block[3].p == nullptr && s.block[3].bytes == 0);
-    CHECK(take_scratch(s, 3, MB, false, d, &a) == 0 && s.block[3].bytes == MB);
+    CHECK(take_scratch(s, 3, 10 * MB, false, false, d, &a) == 0 && s.block[3].bytes == 10 * MB && d.live.count(b));
+    CHECK(take_scratch(s, 3, 11 * MB, false, false, d, &a) == kNoMemory && d.live.count(b) && s.block[3].p == nullptr && s.block[3].bytes == 0);
+    CHECK(take_scratch(s, 3, MB, false, false, d, &a) == 0 && s.block[3].bytes == MB);
+    d.limit = UINT64_MAX;
+    // a slot that may grow during a capture waits for nothing then: what the stream still uses is kept beside what the graph takes
+    const int drains = d.drains;
+    CHECK(take_scratch(s, 4, MB, false, true, d, &a) == 0 && take_scratch(s, 4, 2 * MB, false, true, d, &b) == 0 && !d.live.count(a) && d.drains > drains);
+    const size_t kept = s.kept.size();
+    d.in_capture = true;
+    CHECK(take_scratch(s, 4, 3 * MB, false, true, d, &c) == 0 && d.live.count(b) && s.kept.size() == kept + 1 && s.block[4].in_graph);
+    CHECK(take_scratch(s, 1, 3 * MB, false, true, d, &a) == 0 && s.kept.size() == kept + 1 && s.block[1].in_graph);  // the slot's first block
+    d.in_capture = false;
+    CHECK(take_scratch(s, 4, 16 * MB, false, true, d, &a) == 0 && d.live.count(c) && s.block[4].bytes == 16 * MB);
+    // a growth that fails touches no other slot
+    d.limit = 16 * MB;
+    a = s.block[3].p;
+    CHECK(take_scratch(s, 4, 17 * MB, false, true, d, &b) == kNoMemory && s.block[3].p == a && d.live.count(a));
     s.each([&](void* p) { d.release(p); });
     CHECK(d.live.empty());
     return 0;

@@ -5,6 +5,8 @@ The reference is the fp64 product of the operands as rounded to the 16-bit type;
 (cols + 4) * 2^-24 * sum|h(W) h(x)| (the reference's bound for its own GEMM, tests/unit/vulkan/test_vk_head.cpp:1005-1013)."""
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -54,17 +56,22 @@ def test_gemm_tile_edges(be, checker, t, bf16, m, n, k):
     assert np.all(err <= (k + 4) * 2.0**-24 * (np.abs(hx) @ np.abs(hw).T))
 
 
-def test_gemm_split_scratch_is_not_grown_while_capturing(be, checker):
-    # hidden 2560 x 2048 at 77 tokens splits K on every device this runs on; a stream whose partial-sum scratch has never been grown
-    # captures the unsplit plan instead of failing
+def test_gemm_captured_on_a_stream_that_never_ran_splits(be, checker):
+    # 2560 x 2048 at 77 tokens splits K; captured on a stream without scratch for the splits' sums it has the eager call's plan and bits
     import torch
     t, n, k, m = synth.Q4_K, 2560, 2048, 77
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    plan = capi.GemmPlan()
+    assert be.lib.halo_cuda_gemm_plan(t, n, k, m, sms, 0, ctypes.byref(plan)) == 0 and plan.splits > 1
     w, x = synth.quant_weights(t, n, k, 85, 1), synth.activations(m, k, 85, 2)
     wb, xb = be.import_host_readonly(np.ascontiguousarray(w).view(np.uint8).reshape(-1)), be.import_host_readonly(x)
     yb = be.allocate(m * n * 4)
 
-    def call(st, rows, cols):
-        be.gemv(st, hb.GemvArgs(t, hb.TensorRef.of(wb), hb.TensorRef.of(xb), hb.TensorRef.of(yb), rows, cols, m, capi.GEMM_TCGEN05_F16, allow_gemm=True))
+    def call(st, cols=k, no_scratch=False):
+        a = hb.GemvArgs(t, hb.TensorRef.of(wb), hb.TensorRef.of(xb), hb.TensorRef.of(yb), n, cols, m, capi.GEMM_TCGEN05_F16, allow_gemm=True, no_scratch=no_scratch)
+        before = be.scratch_bytes()
+        be.gemv(st, a)
+        return be.scratch_bytes() - before
 
     def result(st):
         y = np.empty((m, n), np.float32)
@@ -73,25 +80,23 @@ def test_gemm_split_scratch_is_not_grown_while_capturing(be, checker):
         return y
 
     eager, captured = be.create_stream(), be.create_stream()
-    call(eager, n, k)
+    call(eager)
     want = result(eager)
-    # the captured stream has its 16-bit copy of x (same size) from a call that does not split: one W tile of one row, unsplit by the flag
-    a = hb.GemvArgs(t, hb.TensorRef.of(wb), hb.TensorRef.of(xb), hb.TensorRef.of(yb), n, k, m, capi.GEMM_TCGEN05_F16, allow_gemm=True)
-    g = be._gemv_struct(a, "MATMUL", False)
-    g.flags |= capi.FLAG_NO_SCRATCH
-    import ctypes
-    assert be.lib.halo_cuda_gemv(be.ctx, ctypes.byref(g), captured.handle) == 0
+    # the captured stream has its 16-bit copy of x from a call of one block of K, which is never split
+    call(captured, cols=256)
     captured.wait()
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(captured.handle)):
-        call(captured, n, k)
+        assert call(captured) > 0
     be.upload(captured, hb.TensorRef.of(yb), np.full(m * n, -77.0, np.float32))
     captured.wait()
     graph.replay()
     torch.cuda.synchronize()
-    got = result(captured)
+    assert np.array_equal(result(captured), want)
+    # and the plan without splits, which needs none of that scratch
+    assert call(captured, no_scratch=True) == 0
     hw, hx = rounded(checker.dequantize(t, w, n * k).reshape(n, k), False), rounded(x, False)
-    assert np.all(np.abs(got - want) <= 2 * (k + 4) * 2.0**-24 * (np.abs(hx) @ np.abs(hw).T))
+    assert np.all(np.abs(result(captured) - want) <= 2 * (k + 4) * 2.0**-24 * (np.abs(hx) @ np.abs(hw).T))
 
 
 # Shapes whose cheapest tile takes both accumulators (320 to 448 tokens), with and without K splits, and ragged in rows and tokens; the

@@ -201,3 +201,50 @@ def test_i8_batches_are_one_pass_over_the_weights(wtype):
                     assert t.launches == 1, where
                 else:
                     assert t.launches <= 2 and (t.launches == 1 or slices >= 4), where
+
+
+# ---- how the prefill GEMM cuts a call (halo_cuda_gemm_plan) -------------------------------------------------------------------------
+def gemm_plan(wtype: int, rows: int, cols: int, n_vec: int, flags: int = 0, sms: int = 148):
+    p = capi.GemmPlan()
+    assert capi.load().halo_cuda_gemm_plan(wtype, rows, cols, n_vec, sms, flags, C.byref(p)) == 0, capi.last_error()
+    return p
+
+
+@pytest.mark.parametrize("wtype", sorted(MAX_TILE))
+def test_gemm_plans_cover_the_product_and_keep_the_rings_rules(wtype):
+    rng = random.Random(71)
+    for _ in range(600):
+        rows, cols = round(2 ** rng.uniform(0, 17.3)), 256 * round(2 ** rng.uniform(0, 6.9))
+        n_vec, sms = round(2 ** rng.uniform(0, 13)), rng.choice((148, 147, 132, 16, 2))
+        where = f"{rows} x {cols} at {n_vec} tokens on {sms} SMs"
+        p = gemm_plan(wtype, rows, cols, n_vec, sms=sms)
+        tiles = p.row_tiles * p.token_tiles
+        assert p.row_tiles * 256 >= rows > (p.row_tiles - 1) * 256 and p.token_tiles * p.tile_tokens >= n_vec > (p.token_tiles - 1) * p.tile_tokens, where
+        # an accumulator holds 32 to 256 tokens in steps of 32 (the pair's halves are whole 16-row groups), a second one starts beyond 256
+        assert p.tile_tokens % (32 * p.accumulators) == 0 and p.accumulators == (2 if p.tile_tokens > 256 else 1) and p.tile_tokens <= 448, where
+        # a dequantization group fills every fourth stage: its parity wait needs four of them
+        assert 4 <= p.stages <= 8 and 2 <= p.raw_slots <= 3 and p.pairs == sms // 2, where
+        assert p.units == p.whole + (tiles - p.whole) * p.splits and p.whole <= tiles, where
+        if p.splits > 1:
+            assert p.whole % p.pairs == 0 and tiles - p.whole < p.pairs and p.splits <= min(16, cols // 256), where
+        else:
+            assert p.whole == p.units == tiles, where
+        bare = gemm_plan(wtype, rows, cols, n_vec, capi.FLAG_NO_SCRATCH, sms)
+        assert bare.splits == 1 and bare.whole == bare.units == bare.row_tiles * bare.token_tiles, where
+        if p.splits == 1:
+            assert bytes(bare) == bytes(p), where
+
+
+def test_gemm_plan_without_splits_is_made_anew():
+    # 96 tokens a tile on ten of 74 pairs is cheap only with K split; without, more and smaller tiles are
+    p, bare = gemm_plan(synth.Q4_K, 2560, 2048, 77), gemm_plan(synth.Q4_K, 2560, 2048, 77, capi.FLAG_NO_SCRATCH)
+    assert (p.tile_tokens, p.splits > 1) == (96, True) and (bare.tile_tokens, bare.splits) == (32, 1)
+
+
+def test_gemm_plan_refuses_what_it_cannot_describe():
+    lib, p = capi.load(), capi.GemmPlan()
+    assert lib.halo_cuda_gemm_plan(synth.Q4_K, 256, 200, 64, 148, 0, C.byref(p)) == capi.E_MODEL
+    assert lib.halo_cuda_gemm_plan(0, 256, 256, 64, 148, 0, C.byref(p)) == capi.E_UNSUPPORTED
+    assert lib.halo_cuda_gemm_plan(synth.Q4_K, 0, 256, 64, 148, 0, C.byref(p)) < 0
+    assert lib.halo_cuda_gemm_plan(synth.Q4_K, 256, 256, 64, 1, 0, C.byref(p)) < 0
+    assert lib.halo_cuda_gemm_plan(synth.Q4_K, 256, 256, 64, 148, 0, None) == capi.E_API
