@@ -830,8 +830,8 @@ int launch_t(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
     if (int rc = encode_2d(BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, ws, c.cols, c.n_vec, uint64_t{c.cols} * 2, kBK, p.nt / 2u,
                            CU_TENSOR_MAP_SWIZZLE_128B, "x", &xmap))
         return rc;
-    // (the pitch of a one-row matrix is never used, but has to be a valid one)
-    if (int rc = encode_2d(CU_TENSOR_MAP_DATA_TYPE_UINT32, c.w, c.row_bytes / 4u, c.rows, std::max(c.w_stride, c.row_bytes), F::kPitch / 4u, kCtaRows,
+    // (the pitch of a one-row matrix is never used, but has to be a valid one: at least a row, below 2^40)
+    if (int rc = encode_2d(CU_TENSOR_MAP_DATA_TYPE_UINT32, c.w, c.row_bytes / 4u, c.rows, c.rows > 1 ? c.w_stride : c.row_bytes, F::kPitch / 4u, kCtaRows,
                            CU_TENSOR_MAP_SWIZZLE_NONE, "the weight matrix", &wmap))
         return rc;
     cudaLaunchAttribute attr[1];

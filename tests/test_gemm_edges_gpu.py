@@ -123,3 +123,24 @@ def test_gemm_wide_tiles(be, checker, t, n, k, m):
         r = min(640, n - first)
         err = np.abs(y[:, first:first + r].astype(np.float64) - ref[:, :r])
         assert np.all(err <= (k + 4) * 2.0**-24 * mag[:, :r]), f"rows from {first}"
+
+
+@pytest.mark.parametrize("t", (synth.Q4_K, synth.Q8_0))
+def test_gemm_of_one_w_row_has_no_use_for_its_pitch(be, checker, t):
+    # any multiple of 16 is a valid pitch of a matrix of one row, also one the copy engine could not step by
+    k, m = 512, 65
+    w, x = synth.quant_weights(t, 1, k, 97, 1), synth.activations(m, k, 97, 2)
+    st = be.create_stream()
+    wb, variant = be.import_host_readonly(np.ascontiguousarray(w).view(np.uint8).reshape(-1)), capi.GEMM_TCGEN05_F16
+    if t != synth.Q4_K:
+        wb, variant = be.repack(st, t, hb.TensorRef.of(wb), 1, k), capi.GEMM_TCGEN05_F16_R
+    xb, yb = be.import_host_readonly(x), be.allocate(m * 4)
+    got = []
+    for pitch in (0, 16, 1 << 41):
+        g = capi.Gemv(wtype=t, variant_id=variant, w=wb.ptr, w_stride=pitch, x=xb.ptr, y=yb.ptr, rows=1, cols=k, n_vec=m, flags=capi.FLAG_ALLOW_GEMM)
+        assert be.lib.halo_cuda_gemv(be.ctx, ctypes.byref(g), st.handle) == 0, capi.last_error()
+        y = np.empty(m, np.float32)
+        be.download(st, hb.TensorRef.of(yb), y)
+        st.wait()
+        got.append(y)
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2]) and np.any(got[0] != 0)
