@@ -1,5 +1,6 @@
 """The prefill GEMM at the edges of its tiles: W rows around a CTA's 128 and a pair's 256, tokens around the multiples of 32 a tile is
-made of and the 256 / 512 an accumulator or two hold, K of one block and of block counts that splits divide unevenly.
+made of, K of one block and of block counts that splits divide unevenly; and, with the plan of every shape asserted, its states: pairs that
+run several tiles, full accumulators, both accumulators in one tile, whole tiles beside split ones.
 
 The reference is the fp64 product of the operands as rounded to the 16-bit type; the fp32 accumulation may differ from it by
 (cols + 4) * 2^-24 * sum|h(W) h(x)| (the reference's bound for its own GEMM, tests/unit/vulkan/test_vk_head.cpp:1005-1013)."""
@@ -60,9 +61,7 @@ def test_gemm_captured_on_a_stream_that_never_ran_splits(be, checker):
     # 2560 x 2048 at 77 tokens splits K; captured on a stream without scratch for the splits' sums it has the eager call's plan and bits
     import torch
     t, n, k, m = synth.Q4_K, 2560, 2048, 77
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    plan = capi.GemmPlan()
-    assert be.lib.halo_cuda_gemm_plan(t, n, k, m, sms, 0, ctypes.byref(plan)) == 0 and plan.splits > 1
+    assert plan_of(be, t, n, k, m).splits > 1
     w, x = synth.quant_weights(t, n, k, 85, 1), synth.activations(m, k, 85, 2)
     wb, xb = be.import_host_readonly(np.ascontiguousarray(w).view(np.uint8).reshape(-1)), be.import_host_readonly(x)
     yb = be.allocate(m * n * 4)
@@ -99,30 +98,68 @@ def test_gemm_captured_on_a_stream_that_never_ran_splits(be, checker):
     assert np.all(np.abs(result(captured) - want) <= 2 * (k + 4) * 2.0**-24 * (np.abs(hx) @ np.abs(hw).T))
 
 
-# Shapes whose cheapest tile takes both accumulators (320 to 448 tokens), with and without K splits, and ragged in rows and tokens; the
-# first and last W rows against the rounded operands.
-@pytest.mark.parametrize("t,n,k,m", [(synth.Q4_K, 3200, 13824, 259), (synth.Q6_K, 17895, 3328, 280), (synth.Q4_K, 16034, 3584, 282), (synth.Q6_K, 14222, 3840, 346),
-                                     (synth.Q4_0, 9461, 11008, 770)])
-def test_gemm_wide_tiles(be, checker, t, n, k, m):
+def plan_of(be, t, n, k, m):
+    import torch
+    p = capi.GemmPlan()
+    assert be.lib.halo_cuda_gemm_plan(t, n, k, m, torch.cuda.get_device_properties(0).multi_processor_count, 0, ctypes.byref(p)) == 0, capi.last_error()
+    return p
+
+
+def check_tiled_rows(be, checker, t, n, k, m, bf16=False):
+    """W as copies of 640 rows one below the other: every row of the product against the rounded operands at the price of 640."""
     st = be.create_stream()
     block = synth.quant_weights(t, 640, k, 90 + m, 1)
     rows = np.ascontiguousarray(block).view(np.uint8).reshape(640, -1)
     w = np.ascontiguousarray(np.tile(rows, (-(-n // 640), 1))[:n])
     x = synth.activations(m, k, 90 + m, 2)
-    wb, variant = be.import_host_readonly(w.reshape(-1)), capi.GEMM_TCGEN05_F16
+    wb, variant = be.import_host_readonly(w.reshape(-1)), capi.GEMM_TCGEN05_BF16 if bf16 else capi.GEMM_TCGEN05_F16
     if t != synth.Q4_K:
-        wb, variant = be.repack(st, t, hb.TensorRef.of(wb), n, k), capi.GEMM_TCGEN05_F16_R
+        wb, variant = be.repack(st, t, hb.TensorRef.of(wb), n, k), capi.GEMM_TCGEN05_BF16_R if bf16 else capi.GEMM_TCGEN05_F16_R
     xb, yb = be.import_host_readonly(x), be.allocate(m * n * 4)
+    be.upload(st, hb.TensorRef.of(yb), np.full(m * n, np.nan, np.float32))
     be.gemv(st, hb.GemvArgs(t, hb.TensorRef.of(wb), hb.TensorRef.of(xb), hb.TensorRef.of(yb), n, k, m, variant, allow_gemm=True))
     y = np.empty((m, n), np.float32)
     be.download(st, hb.TensorRef.of(yb), y)
     st.wait()
-    hw, hx = rounded(checker.dequantize(t, block, 640 * k).reshape(640, k), False), rounded(x, False)
-    ref, mag = hx @ hw.T, np.abs(hx) @ np.abs(hw).T
+    for b in (wb, xb, yb):
+        b.free()
+    hw, hx = rounded(checker.dequantize(t, block, 640 * k).reshape(640, k), bf16), rounded(x, bf16)
+    ref, bound = hx @ hw.T, (k + 4) * 2.0**-24 * (np.abs(hx) @ np.abs(hw).T)
     for first in range(0, n, 640):
         r = min(640, n - first)
-        err = np.abs(y[:, first:first + r].astype(np.float64) - ref[:, :r])
-        assert np.all(err <= (k + 4) * 2.0**-24 * mag[:, :r]), f"rows from {first}"
+        assert np.all(np.abs(y[:, first:first + r] - ref[:, :r]) <= bound[:, :r]), f"rows from {first}"
+
+
+# (rows, K, tokens) by state and format; rows and tokens ragged
+STATES = {
+    "several tiles a pair": {synth.Q4_K: (580, 256, 1713), synth.Q6_K: (551, 256, 1640), synth.Q8_0: (606, 256, 1629), synth.Q4_0: (572, 256, 1594)},
+    "a full accumulator": {synth.Q4_K: (19693, 1024, 232), synth.Q6_K: (19837, 1024, 228), synth.Q8_0: (26130, 1024, 226), synth.Q4_0: (19258, 1280, 228)},
+    "whole and split": {synth.Q4_K: (20027, 1024, 33), synth.Q6_K: (19170, 768, 33), synth.Q8_0: (20963, 1024, 33), synth.Q4_0: (20083, 1024, 44)},
+    "both accumulators": {synth.Q4_K: (27312, 4352, 582), synth.Q6_K: (27448, 3328, 578), synth.Q8_0: (28303, 4096, 588), synth.Q4_0: (28131, 4864, 577)},
+    "both accumulators, whole and split": {synth.Q4_K: (22057, 4096, 262), synth.Q6_K: (19345, 3584, 265), synth.Q8_0: (19779, 4608, 260), synth.Q4_0: (19109, 5888, 266)},
+}
+
+
+@pytest.mark.parametrize("bf16", (False, True))
+@pytest.mark.parametrize("t", (synth.Q4_K, synth.Q6_K, synth.Q8_0, synth.Q4_0))
+@pytest.mark.parametrize("state", STATES)
+def test_gemm_states(be, checker, state, t, bf16):
+    n, k, m = STATES[state][t]
+    p = plan_of(be, t, n, k, m)
+    assert p.units > p.pairs, "no pair runs a second unit"
+    assert p.accumulators == (2 if "both" in state else 1)
+    assert ((p.whole > 0 and p.splits > 1) if "split" in state else p.splits == 1)
+    if state == "a full accumulator":
+        assert p.tile_tokens == 256
+    check_tiled_rows(be, checker, t, n, k, m, bf16)
+
+
+# Shapes whose cheapest tile takes both accumulators (320 to 448 tokens), with and without K splits, and ragged in rows and tokens
+@pytest.mark.parametrize("t,n,k,m", [(synth.Q4_K, 3200, 13824, 259), (synth.Q6_K, 17895, 3328, 280), (synth.Q4_K, 16034, 3584, 282), (synth.Q6_K, 14222, 3840, 346),
+                                     (synth.Q4_0, 9461, 11008, 770)])
+def test_gemm_wide_tiles(be, checker, t, n, k, m):
+    assert plan_of(be, t, n, k, m).accumulators == 2
+    check_tiled_rows(be, checker, t, n, k, m)
 
 
 @pytest.mark.parametrize("t", (synth.Q4_K, synth.Q8_0))
