@@ -387,7 +387,7 @@ int launch_cfg(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
     return 0;
 }
 
-/// Four x rows a CTA where they fit beside a ring of four rows (K up to about 5400 for Q8_0), else four or two rows beside a ring of two,
+/// Four x rows a CTA where they fit beside a ring of four rows (K up to 5632 for Q8_0, 9728 for Q4_0, 7680 for Q6_K), else four or two rows beside a ring of two,
 /// else one.  A row's arithmetic is the same in all of them.
 template <class F>
 int launch_format(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
@@ -402,14 +402,15 @@ int launch_format(HaloCudaCtx* ctx, const GemvCall& c, cudaStream_t s) {
 /// A lane's 64 weights leave most of a warp without work where K is short, and the kernel that reads both operands from global memory (16 - 32
 /// weights a lane and step) is faster there: over 32 - 34816 rows and 1 - 64 x rows the geometric mean of this form's time over that one's is
 /// Q8_0 1.02 - 1.07 at K = 512 and 0.83 - 0.98 at 640 (256: 1.1 - 1.7), Q4_0 1.0 - 1.1 at 256 and 0.75 - 1.0 at 384, Q6_K 0.85 - 1.44 at 1024
-/// (above 1 from 1024 rows on) and 0.74 - 1.12 at 1280.  The line depends on the type and K alone, since the two add in other orders: a row's bits
+/// (above 1 from 1024 rows on) and 0.74 - 1.12 at 1280.  (Q6_K batches stay slower where a last slot is nearly empty, 10000 x 2304 at four rows 1.5
+/// times, and where one x row fills the memory beside the ring, 1024 x 28672 at sixteen 1.26 times; one row is as fast or four times faster.)  The line depends on the type and K alone, since the two add in other orders: a row's bits
 /// depend neither on the batch nor on how many rows of W a device holds.
 uint32_t least_cols(uint32_t wtype) { return wtype == HALO_CUDA_T_Q8_0 ? 640u : wtype == HALO_CUDA_T_Q4_0 ? 384u : 1280u; }
 
 }  // namespace
 
-/// Raw Q8_0 / Q4_0 / Q6_K rows at even addresses, one x row beside the smallest ring (K up to about 39 000 for Q8_0); a longer or a
-/// shorter K keeps the kernel that reads both operands from global memory.
+/// Raw Q8_0 / Q4_0 / Q6_K rows at even addresses, one x row beside the smallest ring (K up to 40448 for Q8_0, 48640 for Q4_0, 44032 for
+/// Q6_K); a longer or a shorter K keeps the kernel that reads both operands from global memory.
 bool gemv_raw_supports(const GemvCall& c) {
     if (c.cols == 0 || c.rows == 0 || c.n_vec == 0 || reinterpret_cast<uintptr_t>(c.w) % 2 != 0 || c.w_stride % 2 != 0) return false;
     if (reinterpret_cast<uintptr_t>(c.x) % 16 != 0 || c.x_stride % 16 != 0) return false;
