@@ -77,3 +77,37 @@ def test_lm_head_shard_offsets_merge_to_the_full_answer(hz, checker):
         cand = [(-(p[i, 1:2].view(np.float32)[0]), int(p[i, 0])) for p in parts]
         best = min(cand)
         assert best[1] == int(full[i, 0])
+
+
+# Logits whose rows start on 16-byte boundaries (whole chunks of 8192 are read in 16-byte words) or do not (one by one), and a ragged last chunk
+@pytest.mark.parametrize("pad", (0, 1, 2, 3))
+@pytest.mark.parametrize("valid", (0, 3, 8192, 8192 + 7, 3 * 8192 + 2))
+def test_argmax_over_ties_infinities_and_nan(hz, pad, valid):
+    be, st = hz.be, hz.st
+    V, E, stride = 3 * 8192 + 4, 32, 3 * 8192 + 4 + pad
+    rng = np.random.default_rng(5)
+    q = rng.integers(1, 100, V)                       # one code a row, scale 1: logit = code * x[0]
+    q[[5000, 8191, 8192, 9001, V - 1]] = 120          # the largest in every chunk, at a chunk's edges, in the ragged one
+    q[[2, 8195, 8198]] = 110
+    w = np.zeros((V, 34), np.uint8)
+    w[:, :2], w[:, 2] = np.frombuffer(np.float16(1.0).tobytes(), np.uint8), q.astype(np.uint8)
+    head = np.array([1.0, -1.0, np.inf, -np.inf, np.nan, 0.0], np.float32)
+    x = np.zeros((len(head), E), np.float32)
+    x[:, 0] = head
+    wb, xb = be.import_host_readonly(w.reshape(-1)), be.import_host_readonly(x)
+    lb, rb, ib = be.allocate(len(head) * stride * 4), be.allocate(len(head) * 12), be.allocate(len(head) * 4)
+    g = hb.GemvArgs(synth.Q8_0, hb.TensorRef.of(wb), hb.TensorRef.of(xb), hb.TensorRef(lb, 0, 0, stride * 4), V, E, len(head), capi.GEMV_EXACT8)
+    be.lm_head(st, hb.LmHeadArgs(g, hb.TensorRef.of(rb), valid, hb.TensorRef.of(ib), 0))
+    res, ids = np.zeros((len(head), 3), np.uint32), np.zeros(len(head), np.int32)
+    be.download(st, hb.TensorRef.of(rb), res)
+    be.download(st, hb.TensorRef.of(ib), ids)
+    st.wait()
+    limit = valid or V
+    with np.errstate(invalid="ignore"):
+        logits = (q.astype(np.float32) * head[:, None])[:, :limit]
+    for i, h in enumerate(head):
+        if np.isnan(h):
+            assert res[i].tolist() == [0xFFFFFFFF, 0x7FC00000, 1] and ids[i] == 0
+        else:
+            best = int(np.argmax(logits[i]))  # the first of equals, as the sequential scan has it
+            assert res[i].tolist() == [best, int(bits(logits[i, best:best + 1])[0]), 0] and ids[i] == best
