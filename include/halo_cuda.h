@@ -49,7 +49,8 @@ extern "C" {
 
 /* ---- kernel variants of MATMUL (KernelChoice::variant_id, backend.h:173-176).  Ids are explicit
  * and append-only; 0 selects by shape.  "family" groups variants whose rows are bitwise independent
- * of the batch size among themselves (the batch-invariance contract of backend.h:300-304). -------- */
+ * of the batch size among themselves (the batch-invariance contract of backend.h:300-304); family 4, the prefill GEMM that
+ * a caller opts into, is outside of that contract: the order a row is added up in goes with n_vec (halo_cuda_gemm_plan). -------- */
 #define HALO_CUDA_GEMV_DEFAULT 0
 #define HALO_CUDA_GEMV_EXACT8 1       /* bit-identical to the CPU backend (8-lane dot order) */
 #define HALO_CUDA_GEMV_WARP_F32 2     /* fp32 CUDA-core streaming kernel, warp-shuffle reduce */
@@ -69,7 +70,8 @@ extern "C" {
 #define HALO_CUDA_GEMV_FLAG_ALLOW_GEMM 1u /* GemvArgs::allow_gemm: the caller accepts fp16 GEMM numerics */
 #define HALO_CUDA_GEMV_FLAG_NO_SCRATCH 0x80000000u /* never touch context scratch: the tensor-core variants then take their
                                                        statically partitioned kernels (another summation order over K, so the
-                                                       last bits differ from the default; batches run slower) */
+                                                       last bits differ from the default; batches run slower).  The prefill GEMM
+                                                       keeps its 16-bit copy of x in scratch under this flag too; K it never splits then */
 
 typedef struct HaloCudaCtx HaloCudaCtx; /* one per device, opaque */
 typedef void* HaloCudaStream;           /* a cudaStream_t */
@@ -176,10 +178,12 @@ int halo_cuda_ctx_set_peer_wait_polls(HaloCudaCtx* ctx, uint32_t polls);
  * the device; calls on ONE stream reuse that stream's scratch in stream order.  halo_cuda_stream_destroy releases the stream's scratch.
  * A call captured into a CUDA graph holds the address of its stream's scratch: that block stays until the stream or the context is
  * destroyed, also when later calls grow the scratch, so the graph may be replayed (in order with the stream's other work) until then.
+ * Scratch does not grow while its stream is being captured -- run the call once before -- but for the sums of the prefill GEMM's K
+ * splits: a captured prompt has the plan and the bits of the same call made eagerly, whatever the stream ran before.
  * (halo_cuda_lm_head_noalloc is the exception: its fixed array is shared by every call on the GPU.)
  * Bytes of context scratch (staged activations, split-K partials, LM-head logits and argmax partials) the context holds right now:
  * memory the kernels allocated on demand beyond the caller's operands.  Stays 0 for a context that only ever made calls that need
- * none (the exact / fp32 variants, HALO_CUDA_GEMV_FLAG_NO_SCRATCH, halo_cuda_lm_head_noalloc). */
+ * none (the exact / fp32 variants, HALO_CUDA_GEMV_FLAG_NO_SCRATCH without the prefill GEMM, halo_cuda_lm_head_noalloc). */
 int halo_cuda_ctx_scratch_bytes(HaloCudaCtx* ctx, uint64_t* bytes);
 /* Backend::upload / download / copy (backend.h:549-552, 476-481); src of an upload must stay valid until the sync. */
 int halo_cuda_memcpy_h2d_async(HaloCudaCtx* ctx, void* dst, const void* src, uint64_t bytes, HaloCudaStream stream);
