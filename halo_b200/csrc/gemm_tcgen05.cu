@@ -10,7 +10,8 @@
 // Structure: a persistent grid of CTA pairs (clusters of two, one CTA per SM).  A pair's tile is 256 W rows x T tokens, W as the M
 // operand of tcgen05.mma.cta_group::2 (128 rows in each CTA), X as its N operand (each CTA holds half of the tokens), fp32
 // accumulators in TMEM (lane = W row, column = token).  T is a multiple of 32 up to 256 with two accumulators used in turn, so that a
-// tile's epilogue runs under the next tile's MMAs, or a multiple of 64 up to 448 with both accumulators in one tile.
+// tile's epilogue runs under the next tile's MMAs, or a multiple of 64 up to 448 with both accumulators in one tile
+// (Q8_0 up to 320, Q6_K up to 384: what leaves room for four stages beside two blocks of quants).
 // Warps of a CTA (768 threads):
 //   0       TMA: this CTA's half of the 16-bit X tile (64 K elements x T/2 tokens per stage, 128-byte swizzle)
 //   1       TMEM allocation; in the leading CTA the tcgen05.mma issue
