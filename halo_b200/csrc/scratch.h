@@ -47,7 +47,8 @@ int take_scratch(Scratch& set, int slot, uint64_t bytes, bool zeroed, bool while
     if (bytes > b.bytes) {
         uint64_t want = (bytes + kUnit - 1) & ~(kUnit - 1), least = want;
         const bool capturing = driver.capturing(), keep = b.p != nullptr && (b.in_graph || (capturing && while_capturing));
-        if (capturing ? !while_capturing : !keep)  // work already enqueued on this stream may still read the old block
+        // Work already enqueued on this stream may still read a block that is to be released.
+        if (capturing ? !while_capturing : !keep && b.p != nullptr)
             if (int rc = driver.drain()) return rc;
         if (keep) {
             try {

@@ -79,6 +79,8 @@ int main() {
     d.limit = 16 * MB;
     a = s.block[3].p;
     CHECK(take_scratch(s, 4, 17 * MB, false, true, d, &b) == kNoMemory && s.block[3].p == a && d.live.count(a));
+    const int waited = d.drains;  // nor does it wait for the stream again and again, with nothing left to release
+    CHECK(take_scratch(s, 4, 17 * MB, false, true, d, &b) == kNoMemory && d.drains == waited);
     s.each([&](void* p) { d.release(p); });
     CHECK(d.live.empty());
     return 0;
